@@ -56,6 +56,8 @@ NX, NY = 3600, 2400
 # tile shape of the CPU oracle arms; the GPU arm autotunes its own (16x8 is
 # what the autotuner picks on a B200 at 3600x2400)
 TILE_M, TILE_H, GROWTH = 16, 8, 1e10
+# --pass-b names of the library's SEVP_PASS_B_* kinds
+PASS_B_KINDS = {"registers": 0, "staged": 1, "pairs": 2}
 
 
 def parse():
@@ -87,9 +89,10 @@ def parse():
     ap.add_argument("--influence-fp32", default="auto",
                     help="growth limit of the per-group FP32 influence data of the inner "
                          "iterations: a number, 'off', or 'auto' (measured)")
-    ap.add_argument("--pass-b", default="registers", choices=["staged", "registers"],
-                    help="kernel of the FP32 PCG tile pass: shared-memory task stages filled "
-                         "by tensor copies, or per-task register loads")
+    ap.add_argument("--pass-b", default="pairs", choices=["pairs", "staged", "registers"],
+                    help="kernel of the tile passes: two columns per lane, or one column per "
+                         "lane with shared-memory task stages filled by tensor copies, or with "
+                         "per-task register loads")
     ap.add_argument("--resume-dev", type=float, default=0.3,
                     help="largest relative distance between the recursive and the replaced "
                          "residual at which a mixed PCG run resumes (<= 0: never)")
@@ -178,14 +181,15 @@ def measured_peak_hbm():
 
 def ncu_traffic(nx, ny, tiles, kernel="passb"):
     """Per-launch DRAM bytes from the committed ncu summaries (profiles/):
-    the FP32 pass-B kernel ("passb", or "passb_staged" for the kernel with
-    tensor-copied task stages), the Schwarz stage kernel averaged over
+    the FP32 pass-B kernel ("passb_pairs", or "passb" and "passb_staged" for
+    the one-column kernels), the Schwarz stage kernel averaged over
     stages 2 and 3 ("couple") or the one-launch Chebyshev kernel ("cheb");
     None when the summary covers another grid or tile shape (they are
     3600x2400 captures with 16x6 tiles)."""
     if (nx, ny, tuple(tiles)) != (3600, 2400, (16, 6)):
         return None
     name, key = {"passb": ("tile_pass_b_3600x2400.md", "traffic_bytes_per_launch_mixed:"),
+                 "passb_pairs": ("pass_b_pairs_3600x2400.md", "traffic_bytes_per_launch:"),
                  "passb_staged": ("pass_b_staged_3600x2400.md", "traffic_bytes_per_launch:"),
                  "couple": ("schwarz_stages_3600x2400.md", "traffic_bytes_per_launch_avg:"),
                  "cheb": ("cheb_3600x2400.md", "traffic_bytes_per_launch:")}[kernel]
@@ -822,7 +826,7 @@ def run_native(args, world, rank, local, dist):
         base.close()
         solver = SevpSolver(p, tile_m=tiles[0], tile_h=tiles[1], growth_limit=GROWTH,
                             precond_fp32=args.precond_fp32, schwarz=use_sw)
-    solver.set_pass_b_kernel(N.PASS_B_STAGED if args.pass_b == "staged" else N.PASS_B_REGISTERS)
+    solver.set_pass_b_kernel(PASS_B_KINDS[args.pass_b])
     solver.set_resume_check(args.resume_dev)
     stream = solver.stream
     cheb_bounds = None
@@ -1033,9 +1037,9 @@ def run_native(args, world, rank, local, dist):
     # when it is on)
     infl_a = int(solver.influence_bytes() * scale) if args.precond_fp32 else mix_groups[2]
     infl_b = int(solver.schwarz_influence_bytes() * scale)
-    # pass B: x,p,r,q in; x,r,z out (without r.z and z with the Schwarz
-    # preconditioner: z1 out); coefficient planes; influence data
-    b_passb = n * (4 * 4 + 3 * 4 + 4 * ncoef) + infl_a
+    # pass B: r,q in; r,z out (z1 with the Schwarz preconditioner);
+    # coefficient planes; influence data
+    b_passb = n * (2 * 4 + 2 * 4 + 4 * ncoef) + infl_a
     # Schwarz stages, per launch averaged over stage 2 (w in, z2 out) and
     # stage 3 (w, z1, r in, z out): halo rows of w (2 per tile row) and of
     # AT (symmetric storage), coefficient planes, the tiling's influence data
@@ -1047,8 +1051,11 @@ def run_native(args, world, rank, local, dist):
     # coefficient planes; influence data
     b_cheb = n * (4 * 3 + 4 * 3 + 4 * ncoef) + infl_a
     short_tiles = tiles[1] <= 6  # FP32 vectors with tiles up to 6 rows run the short-tile kernel
-    staged = solver.pass_b_kernel_used() == N.PASS_B_STAGED
-    if staged:
+    kind = solver.pass_b_kernel_used()
+    staged = kind == N.PASS_B_STAGED
+    if kind == N.PASS_B_PAIRS:
+        passb_name = "k_tile_pair<float, update, dots> (PCG pass B, two columns per lane)"
+    elif staged:
         passb_name = "k_pass_b_tma (PCG pass B, tensor-copied task stages)"
     else:
         passb_name = ("k_tile_short<float, update, dots>" if short_tiles
@@ -1064,7 +1071,9 @@ def run_native(args, world, rank, local, dist):
     else:
         dom_name = passb_name
         bytes_per_launch, avg_s, dom_n = b_passb, tile_ms / 1e3 / max(tile_n, 1), tile_n
-        traffic = ncu_traffic(p.nx, p.ny, tiles, "passb_staged" if staged else "passb")
+        traffic = ncu_traffic(p.nx, p.ny, tiles,
+                              {N.PASS_B_PAIRS: "passb_pairs",
+                               N.PASS_B_STAGED: "passb_staged"}.get(kind, "passb"))
     achieved = bytes_per_launch / avg_s / 1e9 if dom_n else None
 
     # ---- 64-member ensemble (720x360 each), every launch over all members
@@ -1141,7 +1150,8 @@ def run_native(args, world, rank, local, dist):
             "coefficient_planes": 3 if solver.symmetric else 5,
             "influence_fp32_in_inner_solve": bool(args.precond_fp32),
             "resume_check_max_rel_dev": args.resume_dev,
-            "pass_b_kernel": {N.PASS_B_STAGED: "staged (tensor-copied task stages)",
+            "pass_b_kernel": {N.PASS_B_PAIRS: "pairs (two columns per lane)",
+                              N.PASS_B_STAGED: "staged (tensor-copied task stages)",
                               N.PASS_B_REGISTERS: "registers"}.get(solver.pass_b_kernel_used(),
                                                                     "none"),
             "influence_fp32_growth_limit": mix_limit or None,
@@ -1237,7 +1247,7 @@ def run_profile(args):
         tiles = (16, 6) if args.tiles == "auto" else tuple(int(v) for v in args.tiles.split("x"))
         s = SevpSolver(p, tile_m=tiles[0], tile_h=tiles[1], growth_limit=GROWTH,
                        schwarz=args.precond == "schwarz")
-        s.set_pass_b_kernel(N.PASS_B_STAGED if args.pass_b == "staged" else N.PASS_B_REGISTERS)
+        s.set_pass_b_kernel(PASS_B_KINDS[args.pass_b])
         b = torch.from_numpy(p.b).cuda()
         if args.method == "cheb":
             s.chebyshev_setup(b)

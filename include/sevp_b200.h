@@ -292,18 +292,24 @@ int sevp_set_graphs(sevp_ctx *ctx, int enable);
 #define SEVP_PASS_A_TILES 0
 #define SEVP_PASS_A_COLUMNS 1
 int sevp_set_pass_a_kernel(sevp_ctx *ctx, int kind);
-/* Kernel of the FP32 PCG's tile pass (x += alpha p, r -= alpha q, z = M^-1 r,
- * r.z, r.r) on block-Jacobi tiles of at most 6 rows:
- * SEVP_PASS_B_REGISTERS (default) loads each task's rows and influence
- * matrices into registers when it starts; SEVP_PASS_B_STAGED has every warp keep
- * a shared-memory stage that tensor copies fill with the next task's rows
- * and matrices while it marches the current one, where the tiling and the
- * buffers allow it (tiles 8, 16 or 32 columns wide, nx a multiple of 4,
- * symmetric operator, FP64 influence data; otherwise the register kernel
- * runs).  Both give the same x, r and z bit for bit.  Not part of the
- * reference interface. */
+/* Kernel of the tile passes on the block-Jacobi tiles (r -= alpha q, z =
+ * M^-1 r, r.z, r.r).  SEVP_PASS_B_PAIRS (default) holds two columns per lane,
+ * for FP32 and FP64 vectors, where the operator is symmetric and the
+ * influence data FP64; other cases run the one-column kernels, which the
+ * other two kinds always select:
+ * SEVP_PASS_B_REGISTERS loads each task's rows and influence matrices into
+ * registers when it starts (FP32 vectors, tiles of at most 6 rows; other
+ * tiles march row by row); SEVP_PASS_B_STAGED has, in the FP32 PCG's tile
+ * pass, every warp keep a shared-memory stage that tensor copies fill with
+ * the next task's rows and matrices while it marches the current one, where
+ * the tiling and the buffers allow it (tiles 8, 16 or 32 columns wide and at
+ * most 6 rows high, nx a multiple of 4, symmetric operator, FP64 influence
+ * data; otherwise the register kernel runs).  These two give the same x, r
+ * and z bit for bit; the pairs kernel agrees with them to the marching's
+ * rounding.  Not part of the reference interface. */
 #define SEVP_PASS_B_REGISTERS 0
 #define SEVP_PASS_B_STAGED 1
+#define SEVP_PASS_B_PAIRS 2
 int sevp_set_pass_b_kernel(sevp_ctx *ctx, int kind);
 /* Mixed-precision PCG with block-Jacobi tiles (restart_inner 0): after each
  * FP64 residual the stopped run resumes with the preconditioned residual of
@@ -314,8 +320,8 @@ int sevp_set_pass_b_kernel(sevp_ctx *ctx, int kind);
  * before CG goes on along its last direction.  max_rel_dev <= 0 never
  * resumes.  Not part of the reference interface. */
 int sevp_set_resume_check(sevp_ctx *ctx, double max_rel_dev);
-/* The kernel the context's last FP32 PCG tile pass ran: SEVP_PASS_B_REGISTERS
- * or SEVP_PASS_B_STAGED, -1 before the first.  Test hook; not part of the
+/* The kernel the context's last FP32 PCG tile pass ran: SEVP_PASS_B_REGISTERS,
+ * SEVP_PASS_B_STAGED or SEVP_PASS_B_PAIRS, -1 before the first.  Test hook; not part of the
  * reference interface. */
 int sevp_pass_b_kernel_used(const sevp_ctx *ctx);
 /* One stencil pass on caller device buffers with the context's operator and

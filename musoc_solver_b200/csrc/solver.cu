@@ -12,8 +12,10 @@
 //
 // Per PCG iteration two grid passes are made (the two global reductions of CG
 // force two synchronisation points):
-//   pass A (stencil kernel):  p = z + beta p_old ; q = A p ; partial p.q
-//   pass B (tile kernel):     x += alpha p ; r -= alpha q ; z = M^{-1} r ;
+//   pass A (stencil kernel):  x += alpha p_old (the step of the iteration
+//                             before) ; p = z + beta p_old ; q = A p ;
+//                             partial p.q
+//   pass B (tile kernel):     r -= alpha q ; z = M^{-1} r ;
 //                             partial r.z and r.r
 // (with the Schwarz preconditioner, pass B is three tile passes: the update
 // with the first tiling's solve, then k_tile_couple on the shifted tiling
@@ -165,20 +167,24 @@ struct OpApply {
   __device__ void operator()(double (&)[NV]) {}
 };
 
-// PCG pass A: p = z + beta p_old ; q = A p ; p.q  -> alpha = r.z / p.q
+// PCG pass A: x += alpha p_old when that step is pending ; p = z + beta p_old ;
+// q = A p ; p.q  -> alpha = r.z / p.q
 template <typename V>
 struct OpPassA {
   using T = V;
   static constexpr int NV = 1;
   static constexpr bool kUsesState = true;
   const V *z, *pold;
-  V *pnew, *q;
+  V *pnew, *q, *x;
   SolveState *st;
-  V beta;
-  bool first;
+  V beta, alpha;
+  bool first, step, x_init;
   __device__ void prepare(SolveState *s) {
     beta = (V)s->beta;
     first = (s->beta == 0.0);
+    alpha = (V)s->alpha;
+    step = x != nullptr && s->x_pend;
+    x_init = s->x_init;
   }
   __device__ V value(size_t idx) const {
     V zv = z[idx];
@@ -187,12 +193,16 @@ struct OpPassA {
   __device__ void emit(size_t idx, int, V vc, V av, double (&acc)[NV]) const {
     pnew[idx] = vc;
     q[idx] = av;
+    if (step) x[idx] = fma_rn(alpha, pold[idx], x_init ? x[idx] : V(0));
     acc[0] += (double)vc * (double)av;
   }
   __device__ void operator()(double (&s)[NV]) { PassAFin{st}(s); }
 };
 
-// FP64 residual: x_out = x + d (d optional, FP32 correction); ru = b - A x_out
+// FP64 residual: x_out = x + d (d optional, FP32 correction; with dp, the
+// stopped run's last step alpha dp is added to d first, in FP32 as pass A
+// would have, and d counts as zero while that run never wrote it); ru = b - A
+// x_out
 // with the residual operator; r = w_j ru (w_j the row weight of row j, 1
 // without weights) written as R (double or float, optional).  Sums ||r||^2,
 // ||w b||^2 (the scaled system the PCG recursion works on) and ||ru||^2,
@@ -204,7 +214,7 @@ struct OpResidual {
   static constexpr int NV = 5;
   static constexpr bool kUsesState = false;
   const double *x;
-  const float *d;
+  const float *d, *dp;
   double *xout;
   const double *b;
   R *r;
@@ -221,10 +231,18 @@ struct OpResidual {
   double resume_dev;
   const double *roww;  // row weights (ny) or null
   int abs_mode;        // the outer test is absolute: ||b - A x|| <= tol
-  __device__ void prepare(SolveState *) {}
+  float alpha;
+  bool has_d, has_p;
+  __device__ void prepare(SolveState *s) {
+    has_d = d != nullptr && (dp == nullptr || s->x_init);
+    has_p = dp != nullptr && s->x_pend;
+    alpha = (float)s->alpha;
+  }
   __device__ double value(size_t idx) const {
     double v = x[idx];
-    if (d) v += (double)d[idx];
+    float dv = has_d ? d[idx] : 0.f;
+    if (has_p) dv = fma_rn(alpha, dp[idx], dv);
+    if (has_d || has_p) v += (double)dv;
     return v;
   }
   __device__ void emit(size_t idx, int j, double vc, double av, double (&acc)[NV]) const {
@@ -263,6 +281,8 @@ struct OpResidual {
       st->done = 0;
       st->beta = 0.0;
       st->status = SEVP_OK;
+      st->x_pend = 0;
+      st->x_init = 0;
       // the step the stopped run would have taken next, now on the replaced
       // residual: z of its last pass stays (one step behind r).  Sound only
       // while the recursive residual still tracks the true one; a run that
@@ -284,18 +304,14 @@ struct OpResidual {
 // Inputs of one tile row for one lane (prefetched one row ahead).
 template <typename V>
 struct RowIn {
-  V x, p, r, q;
+  V r, q;
   float cw, cs, cc, ce, cn;
 };
 
 template <typename V, bool UPDATE, bool SYM>
-__device__ __forceinline__ void load_row(RowIn<V> &in, const Coeffs &c, const V *x, const V *p,
-                                         const V *r, const V *q, size_t idx) {
-  if (UPDATE) {
-    in.x = x[idx];
-    in.p = p[idx];
-    in.q = q[idx];
-  }
+__device__ __forceinline__ void load_row(RowIn<V> &in, const Coeffs &c, const V *r, const V *q,
+                                         size_t idx) {
+  if (UPDATE) in.q = q[idx];
   in.r = r[idx];
   if (!SYM) {
     in.cw = __ldg(c.al + idx);
@@ -306,7 +322,7 @@ __device__ __forceinline__ void load_row(RowIn<V> &in, const Coeffs &c, const V 
   in.cn = __ldg(c.at + idx);
 }
 
-// UPDATE: fused x += alpha p, r -= alpha q before preconditioning (pass B).
+// UPDATE: fused r -= alpha q before preconditioning (pass B).
 // DOTS:   accumulate r.z and r.r and finish the iteration on the device.
 // SYM:    symmetric operator: AL and AB are taken from the west lane's AR and
 //         the previous row's AT (inside a tile the couplings that cross the
@@ -315,8 +331,8 @@ __device__ __forceinline__ void load_row(RowIn<V> &in, const Coeffs &c, const V 
 //         FP32 inner solve).
 template <typename V, typename MT, bool UPDATE, bool DOTS, bool SYM>
 __global__ void __launch_bounds__(kTileWarps * 32, SEVP_TILE_MINB)
-    k_tile_apply(TileGeom tg, Coeffs c, const MT *__restrict__ mats, V *x, const V *p, V *r,
-                 const V *q, V *z, SolveState *st, double *partials, unsigned *ticket) {
+    k_tile_apply(TileGeom tg, Coeffs c, const MT *__restrict__ mats, V *r, const V *q, V *z,
+                 SolveState *st, double *partials, unsigned *ticket) {
   if ((DOTS || UPDATE) && st->done) return;
   constexpr bool kChain = sizeof(V) == 4;
   extern __shared__ __align__(16) unsigned char tsm[];
@@ -353,10 +369,10 @@ __global__ void __launch_bounds__(kTileWarps * 32, SEVP_TILE_MINB)
     int t = 0, kb = 0, ke = sub_start(1, hh, nb) - 1;
     RowIn<V> cur{}, nxt{};
     const size_t idx0 = (size_t)j0 * nx + i;
-    if (active) load_row<V, UPDATE, SYM>(cur, c, x, p, r, q, idx0);
+    if (active) load_row<V, UPDATE, SYM>(cur, c, r, q, idx0);
     for (int k = 0; k < hh; ++k) {
       const size_t idx = idx0 + (size_t)k * nx;
-      if (active && k + 1 < hh) load_row<V, UPDATE, SYM>(nxt, c, x, p, r, q, idx + nx);
+      if (active && k + 1 < hh) load_row<V, UPDATE, SYM>(nxt, c, r, q, idx + nx);
       double rv = 0.0;
       double cw, cs;
       if (SYM) {
@@ -377,9 +393,7 @@ __global__ void __launch_bounds__(kTileWarps * 32, SEVP_TILE_MINB)
       const double rcp_k = kChain ? march_rcp(cn) : 0.0;
       if (active) {
         if (UPDATE) {
-          V xn = cur.x + (V)alpha * cur.p;
           V rn = cur.r - (V)alpha * cur.q;
-          x[idx] = xn;
           r[idx] = rn;
           rv = (double)rn;
         } else {
@@ -508,8 +522,8 @@ __global__ void __launch_bounds__(kTileWarps * 32, SEVP_TILE_MINB)
 // rows unrolled.
 template <typename V, typename MT, bool UPDATE, bool DOTS, bool SYM, int HM>
 __global__ void __launch_bounds__(kTileWarps * 32, 2)
-    k_tile_short(TileGeom tg, Coeffs c, const MT *__restrict__ mats, V *x, const V *p, V *r,
-                 const V *q, V *z, SolveState *st, double *partials, unsigned *ticket) {
+    k_tile_short(TileGeom tg, Coeffs c, const MT *__restrict__ mats, V *r, const V *q, V *z,
+                 SolveState *st, double *partials, unsigned *ticket) {
   if ((DOTS || UPDATE) && st->done) return;
   constexpr bool kChain = sizeof(V) == 4;
   __shared__ double dv_all[kTileWarps * 32];
@@ -533,30 +547,23 @@ __global__ void __launch_bounds__(kTileWarps * 32, 2)
     const size_t idx0 = (size_t)j0 * nx + i;
 
     // ---- all loads of the task
-    V rr[HM], xx[UPDATE ? HM : 1], pp[UPDATE ? HM : 1], qq[UPDATE ? HM : 1];
+    V rr[HM], qq[UPDATE ? HM : 1];
     float cc_[HM], ce_[HM], cn_[HM], cw_[SYM ? 1 : HM], cs_[SYM ? 1 : HM];
 #pragma unroll
     for (int k = 0; k < HM; ++k) {
       const bool ok = active && k < hh;
       const size_t id = ok ? idx0 + (size_t)k * nx : 0;
       rr[k] = ok ? r[id] : V(0);
-      if (UPDATE) {
-        xx[k] = ok ? x[id] : V(0);
-        pp[k] = ok ? p[id] : V(0);
-        qq[k] = ok ? q[id] : V(0);
-      }
+      if (UPDATE) qq[k] = ok ? q[id] : V(0);
     }
     load_task_coeffs<SYM, HM>(c, idx0, nx, hh, active, cc_, ce_, cn_, cw_, cs_);
 
-    // row k's right-hand side: the residual, after the fused update
-    // x += alpha p, r -= alpha q
+    // row k's right-hand side: the residual, after the fused r -= alpha q
     auto rhs = [&](int k) -> double {
       if (!active) return 0.0;
       if (UPDATE) {
         const size_t idx = idx0 + (size_t)k * nx;
-        const V xn = xx[k] + (V)alpha * pp[k];
         const V rn = rr[k] - (V)alpha * qq[k];
-        x[idx] = xn;
         r[idx] = rn;
         rr[k] = rn;
       }
@@ -928,6 +935,7 @@ struct Tiling {
   Coeffs c{};                   // the planes its kernels read
   float *d_al = nullptr, *d_ar = nullptr;  // seam-cut AL/AR copies (closed grids, shifted tiling)
   int *d_grp_nb = nullptr;
+  int2 *d_pair_order = nullptr;
   long long *d_moff = nullptr;
   double *d_mats = nullptr;
   float *d_mats32 = nullptr;
@@ -943,8 +951,10 @@ struct Tiling {
   bool built = false;
   void release() {
     for (void *p : {(void *)d_grp_nb, (void *)d_moff, (void *)d_mats, (void *)d_mats32,
-                    (void *)d_al, (void *)d_ar, (void *)d_matsmix, (void *)d_grp_f32})
+                    (void *)d_al, (void *)d_ar, (void *)d_matsmix, (void *)d_grp_f32,
+                    (void *)d_pair_order})
       if (p) cudaFree(p);
+    d_pair_order = nullptr, tg.pair_order = nullptr;
     d_grp_nb = nullptr, d_moff = nullptr, d_mats = nullptr, d_mats32 = nullptr;
     d_al = nullptr, d_ar = nullptr, d_matsmix = nullptr, d_grp_f32 = nullptr;
     tg.grp_f32 = nullptr;
@@ -1038,7 +1048,7 @@ struct sevp_ctx {
   int use_graphs = 1;
   int stencil_rpw = 0;  // rows per CTA of the stencil kernels (0: not chosen yet)
   int pass_a_kernel = SEVP_PASS_A_TILES;
-  int pass_b_kernel = SEVP_PASS_B_REGISTERS;
+  int pass_b_kernel = SEVP_PASS_B_PAIRS;
   int pass_b_used = -1;  // kernel of the last FP32 pass B launch
   cudaStream_t cap_stream = nullptr;
   cudaGraphExec_t inner_graph = nullptr;
@@ -1171,8 +1181,8 @@ static int resident_ctas(K kern, size_t smem, size_t &set_smem, int &slots) {
 }
 
 template <typename V, typename MT, bool UPDATE, bool DOTS, bool SYM>
-static int launch_tile_k(sevp_ctx *ctx, const Tiling &T, const MT *mats, V *x, const V *p, V *r,
-                         const V *q, V *z, int ticket_slot) {
+static int launch_tile_k(sevp_ctx *ctx, const Tiling &T, const MT *mats, V *r, const V *q, V *z,
+                         int ticket_slot) {
   const size_t warps = tile_warps(T.tg);
   const bool short_tiles = sizeof(V) == 4 && T.tg.hmax <= kShortTileRows;
   const size_t smem = short_tiles ? 0 : tile_smem_per_warp(T.tg.hmax) * kTileWarps;
@@ -1188,7 +1198,7 @@ static int launch_tile_k(sevp_ctx *ctx, const Tiling &T, const MT *mats, V *x, c
   if constexpr (sizeof(V) == 4 && std::is_same<MT, double>::value && UPDATE && DOTS && SYM) {
     // PCG pass B with tensor-copied task stages, on the same grid
     if (short_tiles && ctx->pass_b_kernel == SEVP_PASS_B_STAGED) {
-      const PassBLaunch L{T.tg, T.c, mats, x, p, r, q, z, ctx->st, ctx->partials,
+      const PassBLaunch L{T.tg, T.c, mats, r, q, z, ctx->st, ctx->partials,
                           ctx->partials_n, ctx->tickets + ticket_slot, blocks, ctx->stream};
       if (pass_b_tma_eligible(L)) {
         ProfScope ps(ctx, 0);
@@ -1201,34 +1211,47 @@ static int launch_tile_k(sevp_ctx *ctx, const Tiling &T, const MT *mats, V *x, c
     ctx->pass_b_used = SEVP_PASS_B_REGISTERS;
   }
   ProfScope ps(ctx, UPDATE ? 0 : 2);
-  kern<<<blocks, kTileWarps * 32, smem, ctx->stream>>>(T.tg, T.c, mats, x, p, r, q, z, ctx->st,
+  kern<<<blocks, kTileWarps * 32, smem, ctx->stream>>>(T.tg, T.c, mats, r, q, z, ctx->st,
                                                       ctx->partials, ctx->tickets + ticket_slot);
   ctx->launches++;
   SEVP_CUDA_TRY(cudaGetLastError());
   return SEVP_OK;
 }
 
+// Two-column tile pass (tile_pair.cuh).
+template <typename V, bool UPDATE, bool DOTS>
+static int launch_tile_pair(sevp_ctx *ctx, const Tiling &T, V *r, const V *q, V *z,
+                            int ticket_slot) {
+  if (sizeof(V) == 4 && UPDATE && DOTS) ctx->pass_b_used = SEVP_PASS_B_PAIRS;
+  ProfScope ps(ctx, UPDATE ? 0 : 2);
+  const PairLaunch<V> L{T.tg, T.c, T.d_mats, r, q, z, ctx->st, ctx->partials, ctx->partials_n,
+                        ctx->tickets + ticket_slot, ctx->stream, UPDATE, DOTS};
+  ctx->launches++;
+  return tile_pair_launch(L);
+}
+
 // Dispatch: symmetric-coefficient variant when the operator is symmetric;
 // FP32 influence matrices only for FP32 vectors when the solve asks for them.
 template <typename V, bool UPDATE, bool DOTS>
-static int launch_tile(sevp_ctx *ctx, const Tiling &T, V *x, const V *p, V *r, const V *q, V *z,
-                       int ticket_slot) {
+static int launch_tile(sevp_ctx *ctx, const Tiling &T, V *r, const V *q, V *z, int ticket_slot) {
   if constexpr (sizeof(V) == 4) {
     if (ctx->infl32_active && T.d_mats32) {
       if (ctx->sym)
-        return launch_tile_k<V, float, UPDATE, DOTS, true>(ctx, T, T.d_mats32, x, p, r, q, z, ticket_slot);
-      return launch_tile_k<V, float, UPDATE, DOTS, false>(ctx, T, T.d_mats32, x, p, r, q, z, ticket_slot);
+        return launch_tile_k<V, float, UPDATE, DOTS, true>(ctx, T, T.d_mats32, r, q, z, ticket_slot);
+      return launch_tile_k<V, float, UPDATE, DOTS, false>(ctx, T, T.d_mats32, r, q, z, ticket_slot);
     }
-    if (T.d_matsmix) {
+    if (T.d_matsmix && T.f32_groups > 0) {  // without FP32 groups: the FP64 data itself
       const MixMat *mm = reinterpret_cast<const MixMat *>(T.d_matsmix);
       if (ctx->sym)
-        return launch_tile_k<V, MixMat, UPDATE, DOTS, true>(ctx, T, mm, x, p, r, q, z, ticket_slot);
-      return launch_tile_k<V, MixMat, UPDATE, DOTS, false>(ctx, T, mm, x, p, r, q, z, ticket_slot);
+        return launch_tile_k<V, MixMat, UPDATE, DOTS, true>(ctx, T, mm, r, q, z, ticket_slot);
+      return launch_tile_k<V, MixMat, UPDATE, DOTS, false>(ctx, T, mm, r, q, z, ticket_slot);
     }
   }
+  if (ctx->sym && ctx->pass_b_kernel == SEVP_PASS_B_PAIRS && T.tg.hmax <= kPairMaxRows)
+    return launch_tile_pair<V, UPDATE, DOTS>(ctx, T, r, q, z, ticket_slot);
   if (ctx->sym)
-    return launch_tile_k<V, double, UPDATE, DOTS, true>(ctx, T, T.d_mats, x, p, r, q, z, ticket_slot);
-  return launch_tile_k<V, double, UPDATE, DOTS, false>(ctx, T, T.d_mats, x, p, r, q, z, ticket_slot);
+    return launch_tile_k<V, double, UPDATE, DOTS, true>(ctx, T, T.d_mats, r, q, z, ticket_slot);
+  return launch_tile_k<V, double, UPDATE, DOTS, false>(ctx, T, T.d_mats, r, q, z, ticket_slot);
 }
 
 // Tile rows the Schwarz stage kernel holds in registers.
@@ -1291,16 +1314,16 @@ static void schwarz_bufs(sevp_ctx *ctx, V *&s1, V *&s2) {
 }
 
 // z = M^-1 r with the preconditioner the context is set to.  UPDATE fuses
-// x += alpha p, r -= alpha q before it (PCG pass B); DOTS accumulates r.z
+// r -= alpha q before it (PCG pass B); DOTS accumulates r.z
 // and r.r and finishes the iteration on the device.  With the Schwarz
 // preconditioner: z1 = M_a r, z2 = M_b (r - A z1), z = z1 + z2 + M_a (r -
 // A (z1 + z2)), the residuals formed from the tile-boundary couplings.
 template <typename V, bool UPDATE, bool DOTS>
-static int precondition_pass(sevp_ctx *ctx, V *x, const V *p, V *r, const V *q, V *z) {
-  if (!schwarz_on(ctx)) return launch_tile<V, UPDATE, DOTS>(ctx, ctx->ta, x, p, r, q, z, 4);
+static int precondition_pass(sevp_ctx *ctx, V *r, const V *q, V *z) {
+  if (!schwarz_on(ctx)) return launch_tile<V, UPDATE, DOTS>(ctx, ctx->ta, r, q, z, 4);
   V *s1, *s2;
   schwarz_bufs(ctx, s1, s2);
-  int s = launch_tile<V, UPDATE, false>(ctx, ctx->ta, x, p, r, q, s1, 4);
+  int s = launch_tile<V, UPDATE, false>(ctx, ctx->ta, r, q, s1, 4);
   if (s) return s;
   SolveState *st = DOTS ? ctx->st : nullptr;
   s = launch_couple<V, 0>(ctx, ctx->tb, ctx->ta.tg.xs, s1, nullptr, nullptr, s2, st, 4);
@@ -1457,7 +1480,7 @@ extern "C" int sevp_set_pass_a_kernel(sevp_ctx *ctx, int kind) {
 }
 
 extern "C" int sevp_set_pass_b_kernel(sevp_ctx *ctx, int kind) {
-  if (!ctx || (kind != SEVP_PASS_B_REGISTERS && kind != SEVP_PASS_B_STAGED)) return SEVP_BAD_ARG;
+  if (!ctx || kind < SEVP_PASS_B_REGISTERS || kind > SEVP_PASS_B_PAIRS) return SEVP_BAD_ARG;
   ctx->pass_b_kernel = kind;
   drop_inner_graph(ctx);
   return SEVP_OK;
@@ -1578,6 +1601,23 @@ static int build_tiling(sevp_ctx *ctx, Tiling &T, int xs) {
       off = (off + 1) & ~1LL;  // 16-byte aligned start for every tile
     }
   T.mats_elems = off;
+  // the two-column pass's task order (TileGeom::pair_order)
+  const int pc = pair_cols(tg);
+  std::vector<int2> light, order;
+  for (int b = 0; b < tg.ty; ++b)
+    for (int g = 0; g < pc; ++g) {
+      bool costly = tile_height(tg, b) < tg.hmax;
+      for (int h = 2 * g; h < std::min(2 * g + 2, tg.txg); ++h) {
+        const int last = std::min((h + 1) * tg.tpw, tg.tx) - 1;
+        costly = costly || T.grp_nb[(size_t)b * tg.txg + h] > 1 || tile_width(tg, last) < tg.wseg;
+      }
+      (costly ? order : light).push_back(make_int2(b, g));
+    }
+  order.insert(order.end(), light.begin(), light.end());
+  SEVP_CUDA_TRY(cudaMalloc((void **)&T.d_pair_order, sizeof(int2) * order.size()));
+  SEVP_CUDA_TRY(cudaMemcpyAsync(T.d_pair_order, order.data(), sizeof(int2) * order.size(),
+                                cudaMemcpyHostToDevice, ctx->stream));
+  tg.pair_order = T.d_pair_order;
   SEVP_CUDA_TRY(cudaMalloc((void **)&T.d_grp_nb, sizeof(int) * T.grp_nb.size()));
   SEVP_CUDA_TRY(cudaMalloc((void **)&T.d_moff, sizeof(long long) * moff.size()));
   SEVP_CUDA_TRY(cudaMalloc((void **)&T.d_mats, sizeof(double) * std::max<long long>(off, 1)));
@@ -1890,13 +1930,13 @@ extern "C" int sevp_apply(sevp_ctx *ctx, const double *x, double *y) {
 
 extern "C" int sevp_precondition(sevp_ctx *ctx, const double *r, double *z) {
   if (!ctx || !ctx->have_op || !r || !z) return SEVP_BAD_ARG;
-  return precondition_pass<double, false, false>(ctx, nullptr, nullptr, const_cast<double *>(r),
+  return precondition_pass<double, false, false>(ctx, const_cast<double *>(r),
                                                  nullptr, z);
 }
 
 extern "C" int sevp_precondition_f32(sevp_ctx *ctx, const float *r, float *z) {
   if (!ctx || !ctx->have_op || !r || !z) return SEVP_BAD_ARG;
-  return precondition_pass<float, false, false>(ctx, nullptr, nullptr, const_cast<float *>(r),
+  return precondition_pass<float, false, false>(ctx, const_cast<float *>(r),
                                                 nullptr, z);
 }
 
@@ -1910,10 +1950,10 @@ static int read_state(sevp_ctx *ctx) {
 // Residual pass: xout = x + d; r = W (b - A xout) with the residual
 // operator and its row weights; the norms into the state (OpResidual).
 template <typename R>
-static int launch_residual(sevp_ctx *ctx, const double *x, const float *d, double *xout,
-                           const double *b, R *r, int set_inner, double tol2,
+static int launch_residual(sevp_ctx *ctx, const double *x, const float *d, const float *dp,
+                           double *xout, const double *b, R *r, int set_inner, double tol2,
                            double outer2 = 0.0, int abs_mode = 0) {
-  OpResidual<R> op{x, d, xout, b, r, ctx->st, tol2, outer2, set_inner, ctx->resume_dev,
+  OpResidual<R> op{x, d, dp, xout, b, r, ctx->st, tol2, outer2, set_inner, ctx->resume_dev,
                    ctx->have_res ? ctx->roww : nullptr, abs_mode};
   if (ctx->have_res) return launch_stencil_c(ctx, op, 2, ctx->cres, ctx->res_sym);
   return launch_stencil(ctx, op, 2);
@@ -1927,6 +1967,10 @@ __global__ void k_state_init(SolveState *st, double tol2, int max_iter, double *
   s.hist = hist;
   s.hist_cap = hist_cap;
   s.status = SEVP_OK;
+  // the stopped run's last step, for the residual pass that follows
+  s.alpha = st->alpha;
+  s.x_pend = st->x_pend;
+  s.x_init = st->x_init;
   *st = s;
 }
 
@@ -1941,6 +1985,9 @@ __global__ void k_state_keep(SolveState *st, double tol2, int max_iter) {
   s.rz = st->rz;
   s.rz_next = st->rz_next;
   s.keep_dir = 1;
+  s.alpha = st->alpha;
+  s.x_pend = st->x_pend;
+  s.x_init = st->x_init;
   *st = s;
 }
 
@@ -1973,6 +2020,19 @@ __global__ void k_state_from_residual(SolveState *st, double tol2, int abs_mode)
   st->iter = 0;
   st->done = 0;
   st->beta = 0.0;
+  st->x_pend = 0;
+  st->x_init = 1;  // the run adds to the caller's x
+}
+
+// x += alpha p: the pending step of a finished FP64 run (pass A adds the
+// others, see SolveState::x_pend).
+__global__ void k_add_step(const SolveState *st, const double *__restrict__ p,
+                           double *__restrict__ x, size_t n) {
+  if (!st->x_pend) return;
+  const double alpha = st->alpha;
+  for (size_t k = (size_t)blockIdx.x * blockDim.x + threadIdx.x; k < n;
+       k += (size_t)gridDim.x * blockDim.x)
+    x[k] = fma_rn(alpha, p[k], x[k]);
 }
 
 // The outer stopping test on the FP64 residual pass's norms.
@@ -2054,6 +2114,7 @@ static int launch_pass_a(sevp_ctx *ctx, const OpPassA<V> &op) {
                      op.pold,
                      op.pnew,
                      op.q,
+                     op.x,
                      ctx->st,
                      ctx->partials,
                      ctx->partials_n,
@@ -2078,10 +2139,10 @@ static int pcg_loop(sevp_ctx *ctx, V *x, V *r, V *z, V *p0, V *p1, V *q, int che
   V *pp[2] = {p0, p1};
   auto interval = [&](int &cur) -> int {  // check_every iterations of passes A and B
     for (int k = 0; k < check_every; ++k) {
-      OpPassA<V> op{z, pp[cur], pp[cur ^ 1], q, ctx->st};
+      OpPassA<V> op{z, pp[cur], pp[cur ^ 1], q, x, ctx->st};
       int s = launch_pass_a(ctx, op);
       if (s) return s;
-      s = precondition_pass<V, true, true>(ctx, x, pp[cur ^ 1], r, q, z);
+      s = precondition_pass<V, true, true>(ctx, r, q, z);
       if (s) return s;
       cur ^= 1;
     }
@@ -2164,7 +2225,7 @@ static int solve_fp64(sevp_ctx *ctx, const double *b, double *x, const sevp_solv
                                            restart == 0 ? ctx->hist : nullptr, ctx->hist_cap);
     ctx->launches++;
     // r = b - A x
-    int s = launch_residual<double>(ctx, x, nullptr, nullptr, b, ctx->r64, 0, tol2);
+    int s = launch_residual<double>(ctx, x, nullptr, nullptr, nullptr, b, ctx->r64, 0, tol2);
     if (s) return s;
     k_state_from_residual<<<1, 1, 0, ctx->stream>>>(ctx->st, tol2, o->tol_abs);
     ctx->launches++;
@@ -2185,13 +2246,20 @@ static int solve_fp64(sevp_ctx *ctx, const double *b, double *x, const sevp_solv
       break;
     }
     // z = M^{-1} r, rz; then iterate
-    s = precondition_pass<double, false, true>(ctx, nullptr, nullptr, ctx->r64, nullptr, ctx->z64);
+    s = precondition_pass<double, false, true>(ctx, ctx->r64, nullptr, ctx->z64);
     if (s) return s;
     int it = 0;
     s = pcg_loop<double>(ctx, x, ctx->r64, ctx->z64, ctx->p64[0], ctx->p64[1], ctx->q64,
                          std::max(1, o->check_every), &it);
     if (s) return s;
     total += it;
+    if (ctx->h_st->x_pend) {
+      // iteration k writes its search direction into p64[(k + 1) & 1]
+      k_add_step<<<(unsigned)std::min<size_t>((ctx->n + 255) / 256, 148 * 16), 256, 0,
+                   ctx->stream>>>(ctx->st, ctx->p64[it & 1], x, ctx->n);
+      ctx->launches++;
+      SEVP_CUDA_TRY(cudaGetLastError());
+    }
     status = ctx->h_st->status;
     if (status != SEVP_OK && status != SEVP_MAXITER) break;
   }
@@ -2243,6 +2311,7 @@ static int solve_mixed(sevp_ctx *ctx, const double *b, double *x, const sevp_sol
   // residual with its last direction
   const bool keep_cheb = method == SEVP_METHOD_CHEB && !o->restart_inner;
   bool have_dir = false;
+  const float *last_p = nullptr;  // the last PCG run's final direction (its step may be pending)
   for (int refine = 0; refine < 64; ++refine) {
     if (keep && have_dir)
       k_state_keep<<<1, 1, 0, ctx->stream>>>(ctx->st, inner2, std::max(o->max_iter - total, 0));
@@ -2263,10 +2332,10 @@ static int solve_mixed(sevp_ctx *ctx, const double *b, double *x, const sevp_sol
     // a few iterations long and resumed solves took 9 iterations against 5
     const bool resume = keep && have_dir && !schwarz_on(ctx) && ctx->resume_dev > 0.0;
     if (have_d)
-      s = launch_residual<float>(ctx, xa, ctx->d32, xb, b, ctx->r32, resume ? 2 : 1, inner2, outer2,
-                                 o->tol_abs);
+      s = launch_residual<float>(ctx, xa, ctx->d32, last_p, xb, b, ctx->r32, resume ? 2 : 1, inner2,
+                                 outer2, o->tol_abs);
     else
-      s = launch_residual<float>(ctx, xa, nullptr, nullptr, b, ctx->r32, 1, inner2, outer2,
+      s = launch_residual<float>(ctx, xa, nullptr, nullptr, nullptr, b, ctx->r32, 1, inner2, outer2,
                                  o->tol_abs);
     if (s) return s;
     if (have_d) std::swap(xa, xb);
@@ -2289,13 +2358,12 @@ static int solve_mixed(sevp_ctx *ctx, const double *b, double *x, const sevp_sol
       status = SEVP_MAXITER;
       break;
     }
-    // inner solve A d = r32 from d = 0
-    SEVP_CUDA_TRY(cudaMemsetAsync(ctx->d32, 0, ctx->n * 4, ctx->stream));
+    // inner solve A d = r32 from d = 0 (a PCG run writes d with its second
+    // pass A, or leaves its only step to the residual pass)
     int it = 0;
     if (method == SEVP_METHOD_PCG) {
       if (!(resume && ctx->h_st->resumed)) {
-        s = precondition_pass<float, false, true>(ctx, nullptr, nullptr, ctx->r32, nullptr,
-                                                  ctx->z32);
+        s = precondition_pass<float, false, true>(ctx, ctx->r32, nullptr, ctx->z32);
         if (s) return s;
       }
       s = pcg_loop<float>(ctx, ctx->d32, ctx->r32, ctx->z32, ctx->p32[0], ctx->p32[1], ctx->q32,
@@ -2306,7 +2374,9 @@ static int solve_mixed(sevp_ctx *ctx, const double *b, double *x, const sevp_sol
         SEVP_CUDA_TRY(cudaMemcpyAsync(ctx->p32[0], ctx->p32[1], ctx->n * sizeof(float),
                                       cudaMemcpyDeviceToDevice, ctx->stream));
       have_dir = have_dir || it > 0;
+      last_p = ctx->p32[keep ? 0 : (it & 1)];
     } else {
+      SEVP_CUDA_TRY(cudaMemsetAsync(ctx->d32, 0, ctx->n * 4, ctx->stream));
       s = cheb_inner(ctx, std::max(1, o->check_every), &it, keep_cheb && have_dir);
       // launch j writes its direction into p32[(j + 1) & 1]; the next inner
       // solve continues from p32[0]
@@ -2772,7 +2842,7 @@ extern "C" int sevp_nn_features(sevp_ctx *ctx, const double *eta1, const double 
   if (s) return s;
   // the feature is the block-Jacobi preconditioner's response (what the
   // network was trained on), whichever preconditioner the solves use
-  s = launch_tile<double, false, false>(ctx, ctx->ta, nullptr, nullptr, ctx->r64, nullptr, m, 1);
+  s = launch_tile<double, false, false>(ctx, ctx->ta, ctx->r64, nullptr, m, 1);
   if (s) return s;
   SEVP_CUDA_TRY(cudaMemsetAsync(ctx->nn_avg, 0, 3 * nn * sizeof(float), ctx->stream));
   const dim3 pgrid((unsigned)ceil_div(ctx->nx / coarse * coarse, kPackThreads),
@@ -2819,7 +2889,7 @@ extern "C" int sevp_add_launches(sevp_ctx *ctx, int n) {
 extern "C" int sevp_relative_residual(sevp_ctx *ctx, const double *b, const double *x,
                                       double *relres) {
   if (!ctx || !ctx->have_op || !b || !x || !relres) return SEVP_BAD_ARG;
-  int s = launch_residual<double>(ctx, x, nullptr, nullptr, b, (double *)nullptr, 0, 0.0);
+  int s = launch_residual<double>(ctx, x, nullptr, nullptr, nullptr, b, (double *)nullptr, 0, 0.0);
   if (s) return s;
   s = read_state(ctx);
   if (s) return s;
@@ -2964,7 +3034,7 @@ static int pass_a_step(sevp_ctx *ctx, const V *z, const V *pold, double beta, V 
                        double *pq_out) {
   if (!ctx || !ctx->have_op || !z || !pold || !pnew || !q) return SEVP_BAD_ARG;
   k_state_pass_a<<<1, 1, 0, ctx->stream>>>(ctx->st, beta);
-  OpPassA<V> op{z, pold, pnew, q, ctx->st};
+  OpPassA<V> op{z, pold, pnew, q, nullptr, ctx->st};
   int s = launch_pass_a(ctx, op);
   if (!s) s = read_state(ctx);
   if (s) return s;

@@ -36,6 +36,11 @@ struct SolveState {
   // residual was close to the replaced one); 0 when the run restarts its
   // preconditioned residual from the replaced residual
   int resumed;
+  // PCG pass A adds the previous iteration's step alpha p to x (it reads that
+  // p anyway).  x_pend: the last iteration's step is not in x yet (the pass
+  // that ends the run leaves it to the residual pass, or to k_add_step);
+  // x_init: 0 while the run's x counts as zero and has not been written
+  int x_pend, x_init;
   unsigned ticket[4];
   // optional record of the PCG coefficients: alpha_j at hist[2 (j-1)],
   // beta_j at hist[2 (j-1) + 1] for iterations j = 1..hist_cap
@@ -575,6 +580,8 @@ struct PassAFin {
   __device__ void operator()(double (&s)[1]) {
     st->pq = s[0];
     st->iter += 1;
+    if (st->x_pend) st->x_init = 1;  // this pass added the step before
+    st->x_pend = 0;
     if (!isfinite(s[0])) {
       st->status = SEVP_NONFINITE;
       st->done = 1;
@@ -583,20 +590,22 @@ struct PassAFin {
       st->done = 1;
     } else {
       st->alpha = st->rz / s[0];
+      st->x_pend = 1;
       if (st->hist && st->iter <= st->hist_cap) st->hist[2 * (st->iter - 1)] = st->alpha;
     }
   }
 };
 
-// Pass A on TMA-staged tiles (stencil_tma.cu): p = z + beta p_old (z alone
-// when beta = 0), q = A p, alpha = r.z / p.q.
+// Pass A on TMA-staged tiles (stencil_tma.cu): x += alpha p_old when the
+// previous iteration's step is pending (x may be null: no update), p = z +
+// beta p_old (z alone when beta = 0), q = A p, alpha = r.z / p.q.
 template <typename V>
 struct PassALaunch {
   GridDims g;
   Coeffs c;
   int sym;
   const V *z, *pold;
-  V *pnew, *q;
+  V *pnew, *q, *x;
   SolveState *st;
   double *partials;
   size_t partials_n;  // doubles in partials
@@ -611,15 +620,13 @@ template <typename V>
 int pass_a_tma_launch(const PassALaunch<V> &L);
 
 // PCG pass B on FP32 vectors with the task rows and influence matrices
-// brought in by the tensor memory accelerator (tile_tma.cu): x += alpha p,
-// r -= alpha q, z = M^-1 r on the block-Jacobi tiles (symmetric operator,
+// brought in by the tensor memory accelerator (tile_tma.cu): r -= alpha q,
+// z = M^-1 r on the block-Jacobi tiles (symmetric operator,
 // FP64 influence data), r.z and r.r, and the finish of the iteration.
 struct PassBLaunch {
   TileGeom tg;
   Coeffs c;
   const double *mats;
-  float *x;
-  const float *p;
   float *r;
   const float *q;
   float *z;
@@ -636,5 +643,29 @@ struct PassBLaunch {
 bool pass_b_tma_eligible(const PassBLaunch &L);
 // SEVP_BAD_ARG (nothing launched) when not eligible.
 int pass_b_tma_launch(const PassBLaunch &L);
+
+// Tile pass with two columns per lane (tile_pair.cuh): r -= alpha q (update),
+// z = M^-1 r on the block-Jacobi tiles of a symmetric operator with FP64
+// influence data, r.z and r.r and the finish of the iteration (dots).
+template <typename V>
+struct PairLaunch {
+  TileGeom tg;
+  Coeffs c;
+  const double *mats;
+  V *r;
+  const V *q;
+  V *z;
+  SolveState *st;
+  double *partials;
+  size_t partials_n;  // doubles in partials (two per CTA are used)
+  unsigned *ticket;
+  cudaStream_t stream;
+  bool update, dots;
+};
+// Tile rows the kernel holds in registers.
+constexpr int kPairMaxRows = 8;
+template <typename V>
+int tile_pair_launch(const PairLaunch<V> &L);
+
 
 }  // namespace sevp

@@ -1,5 +1,6 @@
-// PCG pass A with TMA-staged tiles: p = z + beta p_old, q = A p and the
-// partial sums of p.q (the pass of k_stencil<OpPassA>, see solver.cu).
+// PCG pass A with TMA-staged tiles: x += alpha p_old (the previous
+// iteration's pending step), p = z + beta p_old, q = A p and the partial sums
+// of p.q (the pass of k_stencil<OpPassA>, see solver.cu).
 //
 // The column-walking k_stencil spends most of its issue slots on address
 // arithmetic, predicated loads and shuffles (about 90 instructions per grid
@@ -84,7 +85,7 @@ template <typename V, bool SYM, int STAGES>
 __global__ void __launch_bounds__(kThreads, 2)
     k_pass_a_tma(const __grid_constant__ Maps maps, GridDims g, const V *__restrict__ z,
                  const V *__restrict__ pold, const float *__restrict__ ar_g, V *pnew, V *q,
-                 SolveState *st, double *partials, unsigned *ticket) {
+                 V *__restrict__ x, SolveState *st, double *partials, unsigned *ticket) {
   using S = Stage<V, SYM>;
   if (st->done) return;
   extern __shared__ __align__(128) unsigned char sm_raw[];
@@ -94,6 +95,12 @@ __global__ void __launch_bounds__(kThreads, 2)
   const int tid = threadIdx.x;
   const V beta = (V)st->beta;
   const bool first = st->beta == 0.0;
+  // the pending step of the iteration before: x += alpha p_old on the own
+  // points (p_old is staged here anyway, so the step costs x's own traffic
+  // and the tile pass needs neither x nor p)
+  const bool step = x != nullptr && st->x_pend;
+  const bool x_init = st->x_init;
+  const V alpha = (V)st->alpha;
   const int nx = g.nx, ny = g.ny;
   const int TX = (nx + kTW - 1) / kTW, TY = (ny + kTH - 1) / kTH, ntile = TX * TY;
   if (tid == 0) {
@@ -140,6 +147,14 @@ __global__ void __launch_bounds__(kThreads, 2)
     float *sat = reinterpret_cast<float *>(sp + S::kOff_at);
     float *sal = reinterpret_cast<float *>(sp + S::kOff_al);
     float *sab = reinterpret_cast<float *>(sp + S::kOff_ab);
+    const int col = x0 + tx;
+    const int r0 = ty * kRowsPerThread;
+    V xv[kRowsPerThread];
+#pragma unroll
+    for (int u = 0; u < kRowsPerThread; ++u) {
+      const int j = j0 + r0 + u;
+      xv[u] = (step && x_init && col < nx && j < ny) ? x[(size_t)j * nx + col] : V(0);
+    }
     if (!mbar_wait(smem_u32(&full[k % STAGES]), (unsigned)(k / STAGES) & 1u)) failed = true;
     if (__syncthreads_or(failed)) {
       failed = true;
@@ -172,8 +187,6 @@ __global__ void __launch_bounds__(kThreads, 2)
         for (int e = tid; e < S::kBW * (kTH + 2); e += kThreads) zb[e] = fma_rn(beta, pb[e], zb[e]);
       __syncthreads();
       // q = A p on the own points; p and q out
-      const int col = x0 + tx;
-      const int r0 = ty * kRowsPerThread;
       V vb = zb[r0 * S::kBW + tx + S::kH];
       V vc = zb[(r0 + 1) * S::kBW + tx + S::kH];
 #pragma unroll
@@ -199,6 +212,7 @@ __global__ void __launch_bounds__(kThreads, 2)
           const size_t gi = (size_t)j * nx + col;
           pnew[gi] = vc;
           q[gi] = av;
+          if (step) x[gi] = fma_rn(alpha, pb[(r + 1) * S::kBW + tx + S::kH], xv[u]);
           acc[0] += (double)vc * (double)av;
         }
         vb = vc;
@@ -300,7 +314,7 @@ int launch(const PassALaunch<V> &L) {
   const int ntile = ((nx + kTW - 1) / kTW) * ((ny + kTH - 1) / kTH);
   const unsigned blocks =
       (unsigned)std::min<size_t>(std::min(ntile, slots), std::max<size_t>(1, L.partials_n / 2));
-  kern<<<blocks, kThreads, smem, L.stream>>>(*mp, L.g, L.z, L.pold, L.c.ar, L.pnew, L.q, L.st,
+  kern<<<blocks, kThreads, smem, L.stream>>>(*mp, L.g, L.z, L.pold, L.c.ar, L.pnew, L.q, L.x, L.st,
                                              L.partials, L.ticket);
   SEVP_CUDA_TRY(cudaGetLastError());
   return SEVP_OK;

@@ -47,6 +47,12 @@ struct TileGeom {
   // [ty * txg] 1 where the group's matrices are stored as FP32 in a
   // per-group-precision copy of the influence data (MixMat); may be null
   const unsigned char *grp_f32;
+  // [ty * pair_cols] the two-column tile pass's warp tasks (x: tile row, y:
+  // pair of warp groups): the costly ones (several sub-blocks, ragged edges)
+  // first, then the others, each in row order.  Warps take strided entries,
+  // so the high-latitude tile rows spread evenly over the warps and none of
+  // them ends the pass.
+  const int2 *pair_order;
 };
 
 __host__ __device__ inline int tile_width(const TileGeom &g, int a) {
@@ -57,6 +63,8 @@ __host__ __device__ inline int tile_height(const TileGeom &g, int b) {
   int h = g.ny - b * g.th;
   return h < g.th ? h : g.th;
 }
+// Pairs of warp groups per tile row.
+__host__ __device__ inline int pair_cols(const TileGeom &g) { return (g.txg + 1) / 2; }
 __host__ __device__ inline int sub_start(int t, int hh, int nb) { return (t * hh) / nb; }
 // Grid column of lane n of tile column a (n < tile_width; 0 otherwise).
 __host__ __device__ inline int tile_col(const TileGeom &g, int a, int n) {

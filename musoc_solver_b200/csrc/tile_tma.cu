@@ -1,15 +1,14 @@
 // PCG pass B with the task data brought in by the tensor memory accelerator:
-// x += alpha p, r -= alpha q, z = M^-1 r on the block-Jacobi tiles, r.z and
-// r.r, and the finish of the iteration (the pass of k_tile_short in
-// solver.cu, operation for operation: x, r and z come out bit-identical).
+// r -= alpha q, z = M^-1 r on the block-Jacobi tiles, r.z and r.r, and the
+// finish of the iteration (the pass of k_tile_short in solver.cu, operation
+// for operation: r and z come out bit-identical).
 //
-// The register kernel loads a task's rows (r, x, p, q and the planes AC, AR,
-// AT) and, after the forward march, its influence matrices from global
+// The register kernel loads a task's rows (r, q and the planes AC, AR, AT) and, after the forward march, its influence matrices from global
 // memory, so every task waits out two memory round trips with only 16 warps
 // per SM to cover them.  Here each warp keeps a shared-memory stage of one
 // task: while it marches task t, the copies of task t + stride are in
 // flight.  Lane 0 issues them:
-//   - the rows, as seven 2-D tensor copies of a 32 x th box (columns
+//   - the rows, as five 2-D tensor copies of a 32 x th box (columns
 //     32 g .. 32 g + 31 of tile group g, so every box starts 16-byte
 //     aligned; points past the grid arrive as zeros), right after the warp
 //     has moved task t's rows from the stage into registers;
@@ -31,9 +30,9 @@ namespace sevp {
 namespace {
 
 constexpr int kHM = kShortTileRows;
-constexpr int kArrays = 7;                          // r, x, p, q, AC, AR, AT
+constexpr int kArrays = 5;                          // r, q, AC, AR, AT
 constexpr uint32_t kArrBytes = kHM * 32 * 4;        // one array's rows of a task
-constexpr uint32_t kRowBytes = kArrays * kArrBytes;  // 128-byte multiple
+constexpr uint32_t kRowBytes = kArrays * kArrBytes;  // 128-byte multiple (768 per array)
 
 __host__ __device__ inline uint32_t mat_bytes(int tm) { return 32u * (uint32_t)tm * 8u; }
 __host__ __device__ inline uint32_t stage_bytes(int tm) {
@@ -44,7 +43,7 @@ __host__ __device__ inline uint32_t copy_bytes(int mw) {
 }
 
 struct RowMaps {
-  CUtensorMap r, x, p, q, ac, ar, at;
+  CUtensorMap r, q, ac, ar, at;
 };
 
 // r.z and r.r as TileFin; a failed wait anywhere reports SEVP_TIMEOUT.
@@ -76,7 +75,7 @@ __device__ __forceinline__ double stage_matvec(const double *dv, int segbase, co
 template <int HM>
 __global__ void __launch_bounds__(kTileWarps * 32, 2)
     k_pass_b_tma(const __grid_constant__ RowMaps maps, TileGeom tg,
-                 const double *__restrict__ mats, float *x, float *r, float *z, SolveState *st,
+                 const double *__restrict__ mats, float *r, float *z, SolveState *st,
                  double *partials, unsigned *ticket) {
   if (st->done) return;
   extern __shared__ __align__(128) unsigned char sm_raw[];
@@ -112,12 +111,10 @@ __global__ void __launch_bounds__(kTileWarps * 32, 2)
     tma::fence_proxy_async();
     tma::mbar_expect_tx(bar_rows, (uint32_t)(kArrays * 32 * tg.th * 4));
     tma::load_2d(wu + 0 * kArrBytes, &maps.r, i0, j0, bar_rows);
-    tma::load_2d(wu + 1 * kArrBytes, &maps.x, i0, j0, bar_rows);
-    tma::load_2d(wu + 2 * kArrBytes, &maps.p, i0, j0, bar_rows);
-    tma::load_2d(wu + 3 * kArrBytes, &maps.q, i0, j0, bar_rows);
-    tma::load_2d(wu + 4 * kArrBytes, &maps.ac, i0, j0, bar_rows);
-    tma::load_2d(wu + 5 * kArrBytes, &maps.ar, i0, j0, bar_rows);
-    tma::load_2d(wu + 6 * kArrBytes, &maps.at, i0, j0, bar_rows);
+    tma::load_2d(wu + 1 * kArrBytes, &maps.q, i0, j0, bar_rows);
+    tma::load_2d(wu + 2 * kArrBytes, &maps.ac, i0, j0, bar_rows);
+    tma::load_2d(wu + 3 * kArrBytes, &maps.ar, i0, j0, bar_rows);
+    tma::load_2d(wu + 4 * kArrBytes, &maps.at, i0, j0, bar_rows);
   };
   auto issue_mats = [&](int b, int grp) {
     uint32_t bytes = 0;
@@ -169,19 +166,17 @@ __global__ void __launch_bounds__(kTileWarps * 32, 2)
     }
     ph_rows ^= 1u;
     rows_pending = false;
-    float rr[HM], xx[HM], pp[HM], qq[HM];
+    float rr[HM], qq[HM];
     float cc_[HM], ce_[HM], cn_[HM], cw_[1], cs_[1];
 #pragma unroll
     for (int k = 0; k < HM; ++k) {
       const bool ok = active && k < hh;
       const int e = k * 32 + lane;
       rr[k] = ok ? srow[0 * HM * 32 + e] : 0.f;
-      xx[k] = ok ? srow[1 * HM * 32 + e] : 0.f;
-      pp[k] = ok ? srow[2 * HM * 32 + e] : 0.f;
-      qq[k] = ok ? srow[3 * HM * 32 + e] : 0.f;
-      cc_[k] = ok ? srow[4 * HM * 32 + e] : 0.f;
-      ce_[k] = ok ? srow[5 * HM * 32 + e] : 0.f;
-      cn_[k] = ok ? srow[6 * HM * 32 + e] : 0.f;
+      qq[k] = ok ? srow[1 * HM * 32 + e] : 0.f;
+      cc_[k] = ok ? srow[2 * HM * 32 + e] : 0.f;
+      ce_[k] = ok ? srow[3 * HM * 32 + e] : 0.f;
+      cn_[k] = ok ? srow[4 * HM * 32 + e] : 0.f;
     }
     __syncwarp();
     if (has_next) {
@@ -197,9 +192,7 @@ __global__ void __launch_bounds__(kTileWarps * 32, 2)
     auto rhs = [&](int k) -> double {
       if (!active) return 0.0;
       const size_t idx = idx0 + (size_t)k * nx;
-      const float xn = xx[k] + (float)alpha * pp[k];
       const float rn = rr[k] - (float)alpha * qq[k];
-      x[idx] = xn;
       r[idx] = rn;
       rr[k] = rn;
       const double rv = (double)rn;
@@ -253,12 +246,12 @@ __global__ void __launch_bounds__(kTileWarps * 32, 2)
   reduce_and_finish<3>(v3, partials, ticket, fin);
 }
 
-// Tensor maps of recent launches (a solve alternates between two p buffers).
+// Tensor maps of recent launches (a few contexts may share the thread).
 struct MapKey {
-  const void *p[7];
+  const void *p[kArrays];
   int nx, ny, th;
   bool operator==(const MapKey &o) const {
-    for (int k = 0; k < 7; ++k)
+    for (int k = 0; k < kArrays; ++k)
       if (p[k] != o.p[k]) return false;
     return nx == o.nx && ny == o.ny && th == o.th;
   }
@@ -274,14 +267,14 @@ thread_local int g_maps_next = 0;
 
 const RowMaps *row_maps(const PassBLaunch &L) {
   const int nx = L.tg.nx, ny = L.tg.ny, th = L.tg.th;
-  const MapKey key{{L.r, L.x, L.p, L.q, L.c.ac, L.c.ar, L.c.at}, nx, ny, th};
+  const MapKey key{{L.r, L.q, L.c.ac, L.c.ar, L.c.at}, nx, ny, th};
   for (auto &e : g_maps)
     if (e.used && e.key == key) return &e.maps;
   auto enc = tma::encoder();
   if (!enc) return nullptr;
   RowMaps m{};
-  const void *src[kArrays] = {L.r, L.x, L.p, L.q, L.c.ac, L.c.ar, L.c.at};
-  CUtensorMap *dst[kArrays] = {&m.r, &m.x, &m.p, &m.q, &m.ac, &m.ar, &m.at};
+  const void *src[kArrays] = {L.r, L.q, L.c.ac, L.c.ar, L.c.at};
+  CUtensorMap *dst[kArrays] = {&m.r, &m.q, &m.ac, &m.ar, &m.at};
   for (int k = 0; k < kArrays; ++k)
     if (!tma::encode(enc, dst[k], src[k], false, nx, ny, 32, th)) return nullptr;
   MapEntry &e = g_maps[g_maps_next];
@@ -300,9 +293,8 @@ bool pass_b_tma_eligible(const PassBLaunch &L) {
   if (tg.th < 1 || tg.th > kHM || tg.hmax != tg.th) return false;
   if (tg.nx % 4 != 0 || tg.nx < 32 || tg.ny < tg.th) return false;
   if (tg.grp_f32 || L.blocks < 1 || (size_t)L.blocks * 3 > L.partials_n) return false;
-  for (const void *p : {(const void *)L.x, (const void *)L.p, (const void *)L.r,
-                        (const void *)L.q, (const void *)L.c.ac, (const void *)L.c.ar,
-                        (const void *)L.c.at, (const void *)L.mats})
+  for (const void *p : {(const void *)L.r, (const void *)L.q, (const void *)L.c.ac,
+                        (const void *)L.c.ar, (const void *)L.c.at, (const void *)L.mats})
     if (!p || !tma::aligned16(p)) return false;
   // the maps are cached: the launch that follows finds them
   return row_maps(L) != nullptr;
@@ -319,7 +311,7 @@ int pass_b_tma_launch(const PassBLaunch &L) {
     SEVP_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     set_smem = smem;
   }
-  kern<<<L.blocks, kTileWarps * 32, smem, L.stream>>>(*mp, L.tg, L.mats, L.x, L.r, L.z, L.st,
+  kern<<<L.blocks, kTileWarps * 32, smem, L.stream>>>(*mp, L.tg, L.mats, L.r, L.z, L.st,
                                                       L.partials, L.ticket);
   SEVP_CUDA_TRY(cudaGetLastError());
   return SEVP_OK;

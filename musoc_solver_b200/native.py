@@ -31,6 +31,7 @@ PASS_A_TILES = 0    # stencil pass on tensor-copied shared-memory tiles
 PASS_A_COLUMNS = 1  # stencil pass walking columns with warp shuffles
 PASS_B_REGISTERS = 0  # tile pass loading each task into registers
 PASS_B_STAGED = 1     # tile pass with tensor-copied shared-memory task stages
+PASS_B_PAIRS = 2      # tile pass with two columns per lane (the default)
 
 GUESS_ZERO, GUESS_PREVIOUS, GUESS_LINEAR, GUESS_LEARNED = 0, 1, 2, 3
 

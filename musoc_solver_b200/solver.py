@@ -396,9 +396,10 @@ class SevpSolver:
         N.check(N.lib().sevp_set_pass_a_kernel(self.h, int(kind)), "sevp_set_pass_a_kernel")
 
     def set_pass_b_kernel(self, kind: int):
-        """Kernel of the FP32 PCG's tile pass: N.PASS_B_REGISTERS (the
-        default) or N.PASS_B_STAGED (tensor-copied task stages, where the
-        tiling allows)."""
+        """Kernel of the tile passes: N.PASS_B_PAIRS (the default: two columns
+        per lane, where the operator is symmetric), or the one-column kernels:
+        N.PASS_B_REGISTERS, or N.PASS_B_STAGED (tensor-copied task stages in
+        the FP32 PCG, where the tiling allows)."""
         N.check(N.lib().sevp_set_pass_b_kernel(self.h, int(kind)), "sevp_set_pass_b_kernel")
 
     def set_resume_check(self, max_rel_dev: float):
