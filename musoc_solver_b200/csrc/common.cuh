@@ -67,6 +67,33 @@ __device__ __forceinline__ T ldg(const T *p) {
 __device__ __forceinline__ double ld_stream(const double *p) { return __ldcs(p); }
 __device__ __forceinline__ float ld_stream(const float *p) { return __ldcs(p); }
 
+// Programmatic dependent launch: a kernel launched with launch_overlapped
+// starts while the stream's kernel before it still runs, once every CTA of
+// that one has called pdl_trigger or ended; it may then prepare and read data
+// that no kernel in flight writes, and calls pdl_wait (the kernel before has
+// ended and its writes are visible) before it touches anything else.  Both
+// are no-ops in an ordinary launch (overlap false).
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() {
+  asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+}
+template <typename... KArgs, typename... Args>
+inline cudaError_t launch_overlapped(void (*kern)(KArgs...), dim3 grid, unsigned threads,
+                                     size_t smem, cudaStream_t stream, bool overlap,
+                                     Args... args) {
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cfg.attrs = &attr;
+  cfg.numAttrs = overlap ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kern, KArgs(args)...);
+}
+
 __host__ __device__ inline int ceil_div(int a, int b) { return (a + b - 1) / b; }
 
 }  // namespace sevp

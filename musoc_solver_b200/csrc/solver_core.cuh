@@ -662,8 +662,10 @@ struct PairLaunch {
   cudaStream_t stream;
   bool update, dots;
 };
-// Tile rows the kernel holds in registers.
-constexpr int kPairMaxRows = 8;
+// Tile rows the kernel holds in registers (taller tiles run its rolled loops
+// on rows staged in shared memory), and the most it takes.
+constexpr int kPairRegRows = 8;
+constexpr int kPairMaxRows = 32;
 template <typename V>
 int tile_pair_launch(const PairLaunch<V> &L);
 

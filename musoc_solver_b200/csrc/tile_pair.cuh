@@ -69,16 +69,16 @@ __device__ __forceinline__ void cp_wait() {
 }
 
 // Copies two neighbouring points into the lane's stage slot: one copy (the
-// pair is 2 sizeof(V) aligned), or one per column inside the tile (d1 is the
-// second one's offset from the first).
+// pair is 2 sizeof(V) aligned), or one per column (d1 is the second one's
+// offset from the first, 0 when it is outside the tile).
 template <typename V>
 __device__ __forceinline__ void fetch_pair(unsigned dst, const V *p, size_t id, long long d1,
-                                           bool vec, bool c0, bool c1) {
+                                           bool vec) {
   if (vec) {
-    if (c0) cp_async<2 * sizeof(V)>(dst, p + id);
+    cp_async<2 * sizeof(V)>(dst, p + id);
   } else {
-    if (c0) cp_async<sizeof(V)>(dst, p + id);
-    if (c1) cp_async<sizeof(V)>(dst + (unsigned)sizeof(V), p + id + d1);
+    cp_async<sizeof(V)>(dst, p + id);
+    cp_async<sizeof(V)>(dst + (unsigned)sizeof(V), p + id + d1);
   }
 }
 template <typename V>
@@ -117,11 +117,12 @@ __global__ void __launch_bounds__(kPairWarps * 32, 2)
     k_tile_pair(TileGeom tg, const float *__restrict__ ac, const float *__restrict__ ar,
                 const float *__restrict__ at, const double *__restrict__ mats, V *r, const V *q,
                 V *z, SolveState *st, double *partials, unsigned *ticket, int vec_ok) {
-  const int done = (DOTS || UPDATE) ? st->done : 0;  // tested once the first copies are under way
+  pdl_trigger();
   constexpr int LPT = W / 2;   // lanes per tile
   constexpr int TPW = 64 / W;  // tiles per warp
   constexpr int DVS = W + 2;   // doubles between the tiles' mat-vec inputs (bank shift)
   constexpr unsigned kV = 64 * sizeof(V), kF = 64 * sizeof(float);  // a staged row
+  constexpr bool kReg = HM <= kPairRegRows;  // full tiles in registers
   extern __shared__ __align__(16) unsigned char psm[];
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   unsigned char *base = psm + pair_smem_per_warp<V, W, HM>(tg.nbmax) * wib;
@@ -140,7 +141,6 @@ __global__ void __launch_bounds__(kPairWarps * 32, 2)
                                           (size_t)tg.nbmax * 1024) +
                seg * DVS;
   double2 *dv2 = reinterpret_cast<double2 *>(dv + n);
-  const V alpha = UPDATE ? (V)st->alpha : V(0);
   const bool vec = vec_ok != 0, quad = vec_ok == 2;
   // FP32 rows as 16-byte copies past L1 (a half warp per row): the 8-byte
   // copies allocate L1 lines, of which too few are left beside the stages
@@ -174,47 +174,60 @@ __global__ void __launch_bounds__(kPairWarps * 32, 2)
     g.d1 = g.c1 ? tile_col(tg, a, n + 1) - i0 : 0;
     g.id0 = (size_t)g.b * tg.th * nx + i0;
   };
-  auto fetch_rows = [&](const Geo &g) {
-    if (quad) {
-      const int col = g.g2 * 64 + (lane & 15) * 4;
-      const size_t id = (size_t)(g.b * tg.th + (lane >> 4)) * nx + col;
+  // The copies take no predicate (a branch each, otherwise): lanes and rows
+  // outside the tile copy a clamped place of the grid, and stage_pair masks
+  // what they brought.  VEC: the vectors r and q; else the three planes.
+  auto fetch = [&](const Geo &g, auto is_vec) {
+    constexpr bool VEC = decltype(is_vec)::value;
+    if (quad && (!VEC || kQuadV)) {
+      // a half warp per row, 16 bytes per lane
+      const int col = min(g.g2 * 64 + (lane & 15) * 4, nx - 4);
+      const size_t row0 = (size_t)g.b * tg.th * nx + col;
       constexpr unsigned kC = 2 * HM * kV;  // the planes follow r and q
-#pragma unroll
+#pragma unroll(kReg ? HM / 2 : 2)
       for (int k = 0; k < HM; k += 2) {
-        if (col < nx && k + (lane >> 4) < g.hh) {
-          const size_t e = id + (size_t)k * nx;
+        if (!kReg && k >= g.hh) break;
+        const size_t e = row0 + (size_t)((unsigned)min(k + (lane >> 4), g.hh - 1)) * (unsigned)nx;
+        if constexpr (VEC) {
           if constexpr (kQuadV) {
             cp_async<16>(uq + k * kF, r + e);
             if (UPDATE) cp_async<16>(uq + (HM + k) * kF, q + e);
           }
+        } else {
           cp_async<16>(uq + kC + k * kF, ac + e);
           cp_async<16>(uq + kC + (HM + k) * kF, ar + e);
           cp_async<16>(uq + kC + (2 * HM + k) * kF, at + e);
         }
       }
-      if constexpr (kQuadV) return;
+      return;
     }
-#pragma unroll
+#pragma unroll(kReg ? HM : 2)
     for (int k = 0; k < HM; ++k) {
-      const bool f0 = g.c0 && k < g.hh, f1 = g.c1 && k < g.hh;
-      const size_t id = g.id0 + (size_t)k * nx;
-      fetch_pair<V>(ur + k * kV, r, id, g.d1, vec, f0, f1);
-      if (UPDATE) fetch_pair<V>(ur + (HM + k) * kV, q, id, g.d1, vec, f0, f1);
-      if (!quad) {
-        fetch_pair<float>(uc + k * kF, ac, id, g.d1, vec, f0, f1);
-        fetch_pair<float>(uc + (HM + k) * kF, ar, id, g.d1, vec, f0, f1);
-        fetch_pair<float>(uc + (2 * HM + k) * kF, at, id, g.d1, vec, f0, f1);
+      if (!kReg && k >= g.hh) break;
+      const size_t id = g.id0 + (size_t)((unsigned)min(k, g.hh - 1)) * (unsigned)nx;
+      if constexpr (VEC) {
+        fetch_pair<V>(ur + k * kV, r, id, g.d1, vec);
+        if (UPDATE) fetch_pair<V>(ur + (HM + k) * kV, q, id, g.d1, vec);
+      } else {
+        fetch_pair<float>(uc + k * kF, ac, id, g.d1, vec);
+        fetch_pair<float>(uc + (HM + k) * kF, ar, id, g.d1, vec);
+        fetch_pair<float>(uc + (2 * HM + k) * kF, at, id, g.d1, vec);
       }
     }
   };
+  auto fetch_planes = [&](const Geo &g) { fetch(g, std::false_type{}); };
+  auto fetch_vectors = [&](const Geo &g) { fetch(g, std::true_type{}); };
   // the lane's two columns of a matrix M (mw x mw)
   auto fetch_mat = [&](const double *M, int mw, bool c0, bool c1) {
     if (mw == W) {
 #pragma unroll
       for (int k = 0; k < W; ++k) cp_async<16>(um + k * 512, M + k * W + n);
     } else if ((mw & 1) == 0) {
-      for (int k = 0; k < mw; ++k)
-        if (c0) cp_async<16>(um + k * 512, M + k * mw + n);
+      if (c0) {
+        const double *p = M + n;
+#pragma unroll 8
+        for (int k = 0; k < mw; ++k, p += mw) cp_async<16>(um + k * 512, p);
+      }
     } else {
       for (int k = 0; k < mw; ++k) {
         if (c0) cp_async<8>(um + k * 512, M + k * mw + n);
@@ -242,6 +255,7 @@ __global__ void __launch_bounds__(kPairWarps * 32, 2)
           s1 += d.y * mb.y;
         }
       } else {
+#pragma unroll 8
         for (int k = 0; k < mw; ++k) {
           const double2 mk = stg[k * 32];
           s0 += dv[k] * mk.x;
@@ -263,9 +277,16 @@ __global__ void __launch_bounds__(kPairWarps * 32, 2)
     locate(nxt, entry(pos));
     if (pos + stride < ntasks) locate(nx1, entry(pos + stride));
     geo(nxt);
-    fetch_rows(nxt);
-    cp_commit();
+    // the planes and the influence data do not change during a solve
+    fetch_planes(nxt);
     fetch_first(nxt);
+  }
+  pdl_wait();
+  const int done = (DOTS || UPDATE) ? st->done : 0;  // tested once the first copies are under way
+  const V alpha = UPDATE ? (V)st->alpha : V(0);
+  if (pos < ntasks) {
+    fetch_vectors(nxt);
+    cp_commit();
     cp_commit();
   }
   if (done) {
@@ -280,7 +301,8 @@ __global__ void __launch_bounds__(kPairWarps * 32, 2)
     const size_t id0 = cur.id0;
     const double *mt = mats + cur.moff;
 
-    const bool full = __all_sync(0xffffffffu, hh == HM && nb == 1 && (mw == W || mw == 0));
+    const bool full =
+        kReg && __all_sync(0xffffffffu, hh == HM && nb == 1 && (mw == W || mw == 0));
     // the task after this one enters the stage's rows, and the ones behind it
     // move up
     auto stage_next = [&]() {
@@ -288,7 +310,8 @@ __global__ void __launch_bounds__(kPairWarps * 32, 2)
       if (more) {
         nxt = nx1;
         geo(nxt);
-        fetch_rows(nxt);
+        fetch_planes(nxt);
+        fetch_vectors(nxt);
       }
       cp_commit();
       if (pos + 2 * stride < ntasks) {
@@ -299,104 +322,109 @@ __global__ void __launch_bounds__(kPairWarps * 32, 2)
     // the staged rows (16-byte row copies serve two lanes)
     cp_wait<1>();
     __syncwarp();
-    if (full) {
-      V r0[HM], r1[HM];
-      float cc0[HM], cc1[HM], ce0[HM], ce1[HM], cn0[HM], cn1[HM], cw0[HM];
-#pragma unroll
-      for (int k = 0; k < HM; ++k) {
-        stage_pair<V>(sr + k * kV, c0, c0, r0[k], r1[k]);
-        if (UPDATE) {
-          V q0, q1;
-          stage_pair<V>(sq + k * kV, c0, c0, q0, q1);
-          r0[k] = fma_rn(-alpha, q0, r0[k]);
-          r1[k] = fma_rn(-alpha, q1, r1[k]);
-        }
-        stage_pair<float>(sc + k * kF, c0, c0, cc0[k], cc1[k]);
-        stage_pair<float>(se + k * kF, c0, c0, ce0[k], ce1[k]);
-        stage_pair<float>(sn + k * kF, c0, c0, cn0[k], cn1[k]);
-      }
-      stage_next();
-      if (UPDATE) {
-#pragma unroll
-        for (int k = 0; k < HM; ++k)
-          store_pair<V>(r, id0 + (size_t)k * nx, d1, vec, c0, c0, r0[k], r1[k]);
-      }
-      // couplings across the tile's edges are dropped; lanes without a tile
-      // march zeros (their north coefficient is one)
-#pragma unroll
-      for (int k = 0; k < HM; ++k) {
-        if (n + 2 >= W) ce1[k] = 0.f;
-        if (!c0) cn0[k] = cn1[k] = 1.f;
-        cw0[k] = __shfl_up_sync(0xffffffffu, ce1[k], 1, LPT);
-        if (n == 0) cw0[k] = 0.f;
-      }
-      auto emit = [&](int k, double z0, double z1) {
-        const V v0 = (V)z0, v1 = (V)z1;
-        store_pair<V>(z, id0 + (size_t)k * nx, d1, vec, c0, c0, v0, v1);
-        if (DOTS) {
-          acc_rz += (double)r0[k] * (double)v0;
-          acc_rz += (double)r1[k] * (double)v1;
-        }
-      };
-      if (DOTS) {
+    bool ran = false;
+    if constexpr (kReg) {
+      if (full) {
+        V r0[HM], r1[HM];
+        float cc0[HM], cc1[HM], ce0[HM], ce1[HM], cn0[HM], cn1[HM], cw0[HM];
 #pragma unroll
         for (int k = 0; k < HM; ++k) {
-          const double a0 = (double)r0[k], a1 = (double)r1[k];
-          acc_rr += a0 * a0;
-          acc_rr += a1 * a1;
-        }
-      }
-      // row k's equation residual with the rows below (zb, zc); the terms
-      // that wait on the neighbour shuffles come last
-      auto row = [&](int k, bool first, bool second, double zb0, double zb1, double zc0,
-                     double zc1, double &q0, double &q1) {
-        double p0 = (double)r0[k], p1 = (double)r1[k];
-        if (!first) {
-          const double zw = __shfl_up_sync(0xffffffffu, zc1, 1, LPT);
-          const double ze = __shfl_down_sync(0xffffffffu, zc0, 1, LPT);
-          if (!second) {
-            p0 -= (double)cn0[k > 0 ? k - 1 : 0] * zb0;
-            p1 -= (double)cn1[k > 0 ? k - 1 : 0] * zb1;
+          stage_pair<V>(sr + k * kV, c0, c0, r0[k], r1[k]);
+          if (UPDATE) {
+            V q0, q1;
+            stage_pair<V>(sq + k * kV, c0, c0, q0, q1);
+            r0[k] = fma_rn(-alpha, q0, r0[k]);
+            r1[k] = fma_rn(-alpha, q1, r1[k]);
           }
-          const double e0 = (double)ce0[k];
-          p0 -= (double)cc0[k] * zc0;
-          p1 -= (double)cc1[k] * zc1;
-          p0 -= e0 * zc1;
-          p1 -= e0 * zc0;
-          p0 -= (double)cw0[k] * zw;
-          p1 -= (double)ce1[k] * ze;
+          stage_pair<float>(sc + k * kF, c0, c0, cc0[k], cc1[k]);
+          stage_pair<float>(se + k * kF, c0, c0, ce0[k], ce1[k]);
+          stage_pair<float>(sn + k * kF, c0, c0, cn0[k], cn1[k]);
         }
-        q0 = p0, q1 = p1;
-      };
-      double zb0 = 0.0, zb1 = 0.0, zc0 = 0.0, zc1 = 0.0, q0, q1;
+        stage_next();
+        if (UPDATE) {
 #pragma unroll
-      for (int k = 0; k < HM; ++k) {
-        row(k, k == 0, k == 1, zb0, zb1, zc0, zc1, q0, q1);
-        if (k < HM - 1) {
+          for (int k = 0; k < HM; ++k)
+            store_pair<V>(r, id0 + (size_t)k * nx, d1, vec, c0, c0, r0[k], r1[k]);
+        }
+        // couplings across the tile's edges are dropped; lanes without a tile
+        // march zeros (their north coefficient is one)
+#pragma unroll
+        for (int k = 0; k < HM; ++k) {
+          if (n + 2 >= W) ce1[k] = 0.f;
+          if (!c0) cn0[k] = cn1[k] = 1.f;
+          cw0[k] = __shfl_up_sync(0xffffffffu, ce1[k], 1, LPT);
+          if (n == 0) cw0[k] = 0.f;
+        }
+        auto emit = [&](int k, double z0, double z1) {
+          const V v0 = (V)z0, v1 = (V)z1;
+          store_pair<V>(z, id0 + (size_t)k * nx, d1, vec, c0, c0, v0, v1);
+          if (DOTS) {
+            acc_rz += (double)r0[k] * (double)v0;
+            acc_rz += (double)r1[k] * (double)v1;
+          }
+        };
+        if (DOTS) {
+#pragma unroll
+          for (int k = 0; k < HM; ++k) {
+            const double a0 = (double)r0[k], a1 = (double)r1[k];
+            acc_rr += a0 * a0;
+            acc_rr += a1 * a1;
+          }
+        }
+        // row k's equation residual with the rows below (zb, zc); the terms
+        // that wait on the neighbour shuffles come last
+        auto row = [&](int k, bool first, bool second, double zb0, double zb1, double zc0,
+                       double zc1, double &q0, double &q1) {
+          double p0 = (double)r0[k], p1 = (double)r1[k];
+          if (!first) {
+            const double zw = __shfl_up_sync(0xffffffffu, zc1, 1, LPT);
+            const double ze = __shfl_down_sync(0xffffffffu, zc0, 1, LPT);
+            if (!second) {
+              p0 -= (double)cn0[k > 0 ? k - 1 : 0] * zb0;
+              p1 -= (double)cn1[k > 0 ? k - 1 : 0] * zb1;
+            }
+            const double e0 = (double)ce0[k];
+            p0 -= (double)cc0[k] * zc0;
+            p1 -= (double)cc1[k] * zc1;
+            p0 -= e0 * zc1;
+            p1 -= e0 * zc0;
+            p0 -= (double)cw0[k] * zw;
+            p1 -= (double)ce1[k] * ze;
+          }
+          q0 = p0, q1 = p1;
+        };
+        double zb0 = 0.0, zb1 = 0.0, zc0 = 0.0, zc1 = 0.0, q0, q1;
+#pragma unroll
+        for (int k = 0; k < HM; ++k) {
+          row(k, k == 0, k == 1, zb0, zb1, zc0, zc1, q0, q1);
+          if (k < HM - 1) {
+            zb0 = zc0, zb1 = zc1;
+            zc0 = q0 * march_rcp((double)cn0[k]);
+            zc1 = q1 * march_rcp((double)cn1[k]);
+          }
+        }
+        __syncwarp();
+        *dv2 = make_double2(q0, q1);
+        __syncwarp();
+        double v0, v1;
+        cp_wait<1>();
+        matvec(W, c0, c0, v0, v1);
+        if (more) fetch_first(nxt);
+        cp_commit();
+        zb0 = 0.0, zb1 = 0.0, zc0 = v0, zc1 = v1;
+        emit(0, zc0, zc1);
+#pragma unroll
+        for (int k = 0; k < HM - 1; ++k) {
+          row(k, false, k == 0, zb0, zb1, zc0, zc1, q0, q1);
           zb0 = zc0, zb1 = zc1;
           zc0 = q0 * march_rcp((double)cn0[k]);
           zc1 = q1 * march_rcp((double)cn1[k]);
+          emit(k + 1, zc0, zc1);
         }
+        ran = true;
       }
-      __syncwarp();
-      *dv2 = make_double2(q0, q1);
-      __syncwarp();
-      double v0, v1;
-      cp_wait<1>();
-      matvec(W, c0, c0, v0, v1);
-      if (more) fetch_first(nxt);
-      cp_commit();
-      zb0 = 0.0, zb1 = 0.0, zc0 = v0, zc1 = v1;
-      emit(0, zc0, zc1);
-#pragma unroll
-      for (int k = 0; k < HM - 1; ++k) {
-        row(k, false, k == 0, zb0, zb1, zc0, zc1, q0, q1);
-        zb0 = zc0, zb1 = zc1;
-        zc0 = q0 * march_rcp((double)cn0[k]);
-        zc1 = q1 * march_rcp((double)cn1[k]);
-        emit(k + 1, zc0, zc1);
-      }
-    } else {
+    }
+    if (!ran) {
       // ---- general path: sub-blocks (the two halves of the warp may have
       // different counts), short tiles, narrow last tiles.  Rolled loops on
       // the staged rows (unrolled, its code ran out of the instruction cache
@@ -424,9 +452,14 @@ __global__ void __launch_bounds__(kPairWarps * 32, 2)
           acc_rr += (double)bv * (double)bv;
         }
       }
-      // row k as in the full path, and its reciprocals of AT
-      auto row = [&](int k, double zb0, double zb1, double zc0, double zc1, double &q0, double &q1,
-                     double &i0, double &i1) {
+      // Row k's coefficients and right-hand side, converted, and its
+      // reciprocals of AT: taken one row ahead of the march, so that only the
+      // shuffles, one multiply-add and a multiply are on its chain.
+      struct RowC {
+        double s0, s1, f0, f1, e0, e1, w0, i0, i1, p0, p1;
+      };
+      auto take = [&](int k) {
+        RowC c;
         float f0, f1, s0 = 0.f, s1 = 0.f, n0, n1, e0, e1;
         stage_pair<float>(sc + k * kF, c0, c1, f0, f1);
         stage_pair<float>(se + k * kF, c1, n + 2 < mw, e0, e1);
@@ -434,35 +467,43 @@ __global__ void __launch_bounds__(kPairWarps * 32, 2)
         if (k > 0) stage_pair<float>(sn + (k - 1) * kF, c0, c1, s0, s1);
         float w0 = __shfl_up_sync(0xffffffffu, e1, 1, LPT);
         if (n == 0) w0 = 0.f;
+        c.s0 = (double)s0, c.s1 = (double)s1, c.f0 = (double)f0, c.f1 = (double)f1;
+        c.e0 = (double)e0, c.e1 = (double)e1, c.w0 = (double)w0;
+        c.p0 = (double)wr[k * kR], c.p1 = (double)wr[k * kR + 1];
+        c.i0 = march_rcp(c0 ? (double)n0 : 1.0);
+        c.i1 = march_rcp(c1 ? (double)n1 : 1.0);
+        return c;
+      };
+      auto row = [&](const RowC &c, double zb0, double zb1, double zc0, double zc1, double &q0,
+                     double &q1) {
         const double zw = __shfl_up_sync(0xffffffffu, zc1, 1, LPT);
         const double ze = __shfl_down_sync(0xffffffffu, zc0, 1, LPT);
-        double p0 = (double)wr[k * kR], p1 = (double)wr[k * kR + 1];
-        p0 -= (double)s0 * zb0;
-        p1 -= (double)s1 * zb1;
-        p0 -= (double)f0 * zc0;
-        p1 -= (double)f1 * zc1;
-        p0 -= (double)e0 * zc1;
-        p1 -= (double)e0 * zc0;
-        p0 -= (double)w0 * zw;
-        p1 -= (double)e1 * ze;
+        double p0 = c.p0 - c.s0 * zb0, p1 = c.p1 - c.s1 * zb1;
+        p0 -= c.f0 * zc0;
+        p1 -= c.f1 * zc1;
+        p0 -= c.e0 * zc1;
+        p1 -= c.e0 * zc0;
+        p0 -= c.w0 * zw;
+        p1 -= c.e1 * ze;
         q0 = p0, q1 = p1;
-        i0 = march_rcp(c0 ? (double)n0 : 1.0);
-        i1 = march_rcp(c1 ? (double)n1 : 1.0);
       };
       {
-        double zb0 = 0.0, zb1 = 0.0, zc0 = 0.0, zc1 = 0.0, q0, q1, i0, i1;
+        double zb0 = 0.0, zb1 = 0.0, zc0 = 0.0, zc1 = 0.0, q0, q1;
         int t = 0, kb = 0, ke = sub_start(1, hh, nb) - 1;
+        RowC c = take(0);
 #pragma unroll 1
         for (int k = 0; k < hh; ++k) {
+          const RowC cn = take(min(k + 1, hh - 1));
           if (k == kb) {
             zc0 = zc1 = 0.0;
             zin[t * 32] = make_double2(zb0, zb1);
           }
-          row(k, zb0, zb1, zc0, zc1, q0, q1, i0, i1);
+          row(c, zb0, zb1, zc0, zc1, q0, q1);
           const bool last = k == ke, fix = last && t < nb - 1;
           if (last) rho[t * 32] = make_double2(q0, q1);
           zb0 = zc0, zb1 = zc1;
-          if (!last) zc0 = q0 * i0, zc1 = q1 * i1;
+          if (!last) zc0 = q0 * c.i0, zc1 = q1 * c.i1;
+          c = cn;
           if (__any_sync(0xffffffffu, fix)) {
             __syncwarp();
             *dv2 = make_double2(q0, q1);
@@ -525,10 +566,12 @@ __global__ void __launch_bounds__(kPairWarps * 32, 2)
           }
           cp_commit();
         }
-        double zc0 = v0, zc1 = v1, q0, q1, i0, i1;
+        double zc0 = v0, zc1 = v1, q0, q1;
         const int k_lo = __reduce_min_sync(0xffffffffu, kb), k_hi = __reduce_max_sync(0xffffffffu, ke);
+        RowC c = take(k_lo);
 #pragma unroll 1
         for (int k = k_lo; k <= k_hi; ++k) {
+          const RowC cn = take(min(k + 1, hh - 1));
           const bool in = on && k >= kb && k <= ke;
           if (in) {
             const V u0 = (V)zc0, u1 = (V)zc1;
@@ -538,11 +581,12 @@ __global__ void __launch_bounds__(kPairWarps * 32, 2)
               acc_rz += (double)wr[k * kR + 1] * (double)u1;
             }
           }
-          row(k, zb0, zb1, zc0, zc1, q0, q1, i0, i1);
+          row(c, zb0, zb1, zc0, zc1, q0, q1);
           if (in && k < ke) {
             zb0 = zc0, zb1 = zc1;
-            zc0 = q0 * i0, zc1 = q1 * i1;
+            zc0 = q0 * c.i0, zc1 = q1 * c.i1;
           }
+          c = cn;
         }
         vn0 = v0, vn1 = v1;
       }
@@ -564,31 +608,41 @@ int tile_pair_launch_k(const PairLaunch<V> &L) {
   auto kern = k_tile_pair<V, W, HM, UPDATE, DOTS>;
   const TileGeom &tg = L.tg;
   const size_t per_warp = pair_smem_per_warp<V, W, HM>(tg.nbmax);
-  // resident CTAs of the last shared-memory size, per device (contexts in
-  // several threads may differ in sub-block counts)
+  // CTA size (in warps) with the most resident warps, and its resident CTAs,
+  // for the last shared-memory size (contexts in several threads may differ
+  // in sub-block counts)
   static std::mutex mu;
   static size_t set_smem = 0;
-  static int slots = 0, sms = 0;
-  int use_slots, use_sms;
+  static int best_warps = 1, slots = 1, sms = 1;
+  int use_warps, use_slots, use_sms;
   {
     std::lock_guard<std::mutex> lock(mu);
     if (set_smem != per_warp) {
-      int per_sm = 0, dev = 0;
-      SEVP_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)pair_smem_per_warp<V, W, HM>(HM) * kPairWarps));
-      SEVP_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kPairWarps * 32,
-                                                                  per_warp * kPairWarps));
+      int dev = 0, optin = 0, best = 0;
       SEVP_CUDA_TRY(cudaGetDevice(&dev));
       SEVP_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-      slots = std::max(1, per_sm) * sms;
+      SEVP_CUDA_TRY(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+      const size_t room = (size_t)optin - 1024;  // static shared memory of the sums
+      SEVP_CUDA_TRY(
+          cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)room));
+      for (int w = kPairWarps; w >= 1; --w) {
+        int per_sm = 0;
+        if (per_warp * w > room) continue;
+        SEVP_CUDA_TRY(
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, w * 32, per_warp * w));
+        if (per_sm * w > best) best = per_sm * w, best_warps = w, slots = per_sm * sms;
+      }
+      if (!best) {
+        sevp_internal_set_message("tile pass: a warp's rows do not fit the shared memory");
+        return SEVP_BAD_ARG;
+      }
       set_smem = per_warp;
     }
-    use_slots = slots, use_sms = sms;
+    use_warps = best_warps, use_slots = slots, use_sms = sms;
   }
   const long long ntasks = (long long)tg.ty * pair_cols(tg);
   // few tasks: fewer warps per CTA, so that they spread over the SMs
-  const int warps =
-      (int)std::min<long long>(kPairWarps, std::max<long long>(1, ntasks / use_sms));
+  const int warps = (int)std::min<long long>(use_warps, std::max<long long>(1, ntasks / use_sms));
   const long long want = std::min<long long>((ntasks + warps - 1) / warps, use_slots);
   const unsigned blocks =
       (unsigned)std::max<long long>(1, std::min<long long>(want, (long long)(L.partials_n / 2)));
@@ -601,10 +655,11 @@ int tile_pair_launch_k(const PairLaunch<V> &L) {
   bool quad = vec && tg.nx % 4 == 0 && tg.tm == W && tg.xs == 0;
   for (int k = 0; k < 3; ++k)
     quad = quad && ((uintptr_t)vp[k] & 15) == 0 && ((uintptr_t)cp[k] & 15) == 0;
-  kern<<<blocks, warps * 32, per_warp * warps, L.stream>>>(tg, L.c.ac, L.c.ar, L.c.at, L.mats, L.r,
-                                                           L.q, L.z, L.st, L.partials, L.ticket,
-                                                           quad ? 2 : (vec ? 1 : 0));
-  SEVP_CUDA_TRY(cudaGetLastError());
+  // a solve's kernels only: the planes are read before the kernel ahead has
+  // ended, and outside a solve that kernel may be the caller's, writing them
+  SEVP_CUDA_TRY(launch_overlapped(kern, blocks, warps * 32, per_warp * warps, L.stream,
+                                  UPDATE || DOTS, tg, L.c.ac, L.c.ar, L.c.at, L.mats, L.r, L.q, L.z, L.st, L.partials,
+                                  L.ticket, quad ? 2 : (vec ? 1 : 0)));
   return SEVP_OK;
 }
 
@@ -618,16 +673,18 @@ int tile_pair_launch_w(const PairLaunch<V> &L) {
   return tile_pair_launch_k<V, W, HM, false, false>(L);
 }
 
+template <typename V, int HM>
+int tile_pair_launch_h(const PairLaunch<V> &L) {
+  if (L.tg.wseg == 8) return tile_pair_launch_w<V, 8, HM>(L);
+  if (L.tg.wseg == 16) return tile_pair_launch_w<V, 16, HM>(L);
+  return tile_pair_launch_w<V, 32, HM>(L);
+}
 template <typename V>
 int tile_pair_launch_any(const PairLaunch<V> &L) {
-  if (L.tg.hmax <= 6) {
-    if (L.tg.wseg == 8) return tile_pair_launch_w<V, 8, 6>(L);
-    if (L.tg.wseg == 16) return tile_pair_launch_w<V, 16, 6>(L);
-    return tile_pair_launch_w<V, 32, 6>(L);
-  }
-  if (L.tg.wseg == 8) return tile_pair_launch_w<V, 8, 8>(L);
-  if (L.tg.wseg == 16) return tile_pair_launch_w<V, 16, 8>(L);
-  return tile_pair_launch_w<V, 32, 8>(L);
+  if (L.tg.hmax <= 6) return tile_pair_launch_h<V, 6>(L);
+  if (L.tg.hmax <= 8) return tile_pair_launch_h<V, 8>(L);
+  if (L.tg.hmax <= 16) return tile_pair_launch_h<V, 16>(L);
+  return tile_pair_launch_h<V, 32>(L);
 }
 
 }  // namespace sevp

@@ -1,8 +1,8 @@
 """The two-column tile pass (SEVP_PASS_B_PAIRS) at the sizes where its mapping
 can go wrong: every lane-segment width (8, 16, 32 columns) full and narrower,
 odd tile widths and odd grids (no vector copies), narrow last tiles and short
-last tile rows, tile heights below, at and between the register heights (6
-and 8), sub-block counts that differ between the two halves of a warp, one
+last tile rows, tile heights below, at, between and above the register heights
+(6 and 8), sub-block counts that differ between the two halves of a warp, one
 tile per grid, and caller buffers that are aligned to one value only.
 
 z = M^-1 r against the CPU oracle's tile solve.  Tolerances, of max|z|: 1e-8
@@ -43,6 +43,10 @@ CASES = [
     (120, 60, 12, 6, 1e2),    # many sub-blocks
     (33, 17, 16, 6, 1e3),
     (7, 3, 8, 6, 1e6),        # one partial tile
+    (128, 64, 16, 16, 1e6),   # rows staged in shared memory
+    (131, 65, 16, 9, 1e3),
+    (96, 96, 24, 24, 1e6),
+    (150, 70, 32, 32, 1e4),
 ]
 
 
