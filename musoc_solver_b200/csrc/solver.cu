@@ -199,6 +199,13 @@ struct OpPassA {
   __device__ void operator()(double (&s)[NV]) { PassAFin{st}(s); }
 };
 
+// The outer stopping test on an FP64 residual pass's norms ||b - A x||^2 and
+// ||b||^2 (the same operations on the device and on the host).
+__host__ __device__ inline bool meets_tol(double rr, double bb, double tol, int abs_mode) {
+  if (abs_mode) return sqrt(rr) <= tol;
+  return bb == 0.0 || sqrt(rr / bb) <= tol;
+}
+
 // FP64 residual: x_out = x + d (d optional, FP32 correction; with dp, the
 // stopped run's last step alpha dp is added to d first, in FP32 as pass A
 // would have, and d counts as zero while that run never wrote it); ru = b - A
@@ -223,6 +230,10 @@ struct OpResidual {
   // (safety * outer tolerance)^2: the inner solve need not go below it; a
   // relative tolerance (of ||b||) unless abs_mode
   double outer2;
+  // the outer test's tolerance: a residual that meets it (or is not finite)
+  // marks the inner run done before it starts, so that its first launches can
+  // be queued behind this pass without waiting for the norms
+  double tol;
   // 1: also initialise the inner FP32 solve state; 2: the same for a PCG run
   // that resumes on this residual (beta from the stopped run's last two r.z)
   // when the stopped run's recursive residual, still in r, is within
@@ -296,7 +307,12 @@ struct OpResidual {
         st->resumed = 1;
       }
     }
-    if (!isfinite(s[0]) || !isfinite(s[2]) || !isfinite(s[3])) st->status = SEVP_NONFINITE;
+    if (!isfinite(s[0]) || !isfinite(s[2]) || !isfinite(s[3])) {
+      st->status = SEVP_NONFINITE;
+      if (set_inner) st->done = 1;
+    } else if (set_inner && meets_tol(s[2], s[3], tol, abs_mode)) {
+      st->done = 1;
+    }
   }
 };
 
@@ -322,7 +338,8 @@ __device__ __forceinline__ void load_row(RowIn<V> &in, const Coeffs &c, const V 
   in.cn = __ldg(c.at + idx);
 }
 
-// UPDATE: fused r -= alpha q before preconditioning (pass B).
+// UPDATE: fused r -= alpha q before preconditioning (pass B).  DOTS without
+//         UPDATE starts a run, and is skipped by one that resumes.
 // DOTS:   accumulate r.z and r.r and finish the iteration on the device.
 // SYM:    symmetric operator: AL and AB are taken from the west lane's AR and
 //         the previous row's AT (inside a tile the couplings that cross the
@@ -333,7 +350,7 @@ template <typename V, typename MT, bool UPDATE, bool DOTS, bool SYM>
 __global__ void __launch_bounds__(kTileWarps * 32, SEVP_TILE_MINB)
     k_tile_apply(TileGeom tg, Coeffs c, const MT *__restrict__ mats, V *r, const V *q, V *z,
                  SolveState *st, double *partials, unsigned *ticket) {
-  if ((DOTS || UPDATE) && st->done) return;
+  if ((DOTS || UPDATE) && (st->done || (!UPDATE && st->resumed))) return;
   constexpr bool kChain = sizeof(V) == 4;
   extern __shared__ __align__(16) unsigned char tsm[];
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
@@ -524,7 +541,7 @@ template <typename V, typename MT, bool UPDATE, bool DOTS, bool SYM, int HM>
 __global__ void __launch_bounds__(kTileWarps * 32, 2)
     k_tile_short(TileGeom tg, Coeffs c, const MT *__restrict__ mats, V *r, const V *q, V *z,
                  SolveState *st, double *partials, unsigned *ticket) {
-  if ((DOTS || UPDATE) && st->done) return;
+  if ((DOTS || UPDATE) && (st->done || (!UPDATE && st->resumed))) return;
   constexpr bool kChain = sizeof(V) == 4;
   __shared__ double dv_all[kTileWarps * 32];
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
@@ -1952,8 +1969,8 @@ static int read_state(sevp_ctx *ctx) {
 template <typename R>
 static int launch_residual(sevp_ctx *ctx, const double *x, const float *d, const float *dp,
                            double *xout, const double *b, R *r, int set_inner, double tol2,
-                           double outer2 = 0.0, int abs_mode = 0) {
-  OpResidual<R> op{x, d, dp, xout, b, r, ctx->st, tol2, outer2, set_inner, ctx->resume_dev,
+                           double outer2 = 0.0, int abs_mode = 0, double tol = 0.0) {
+  OpResidual<R> op{x, d, dp, xout, b, r, ctx->st, tol2, outer2, tol, set_inner, ctx->resume_dev,
                    ctx->have_res ? ctx->roww : nullptr, abs_mode};
   if (ctx->have_res) return launch_stencil_c(ctx, op, 2, ctx->cres, ctx->res_sym);
   return launch_stencil(ctx, op, 2);
@@ -2012,13 +2029,16 @@ __global__ void k_state_keep_cheb(SolveState *st, double tol2, int max_iter) {
 // (row-scaled) residual must fall by the factor the outer test still needs,
 // target / ||b - A x||^2 with target = tol^2 ||b||^2 (relative test) or
 // tol^2 (absolute test).
-__global__ void k_state_from_residual(SolveState *st, double tol2, int abs_mode) {
+__global__ void k_state_from_residual(SolveState *st, double tol, int abs_mode) {
+  const double tol2 = tol * tol;
   const double target = abs_mode ? tol2 : tol2 * st->bb64;
   st->tol2 = st->rr64 > 0.0 ? target / st->rr64 : tol2;
   st->bb = st->rr64w;
   st->rr = st->rr64w;
   st->iter = 0;
-  st->done = 0;
+  // a residual that meets the tolerance, or is not finite, starts no run
+  st->done = !isfinite(st->rr64) || !isfinite(st->bb64) ||
+             meets_tol(st->rr64, st->bb64, tol, abs_mode);
   st->beta = 0.0;
   st->x_pend = 0;
   st->x_init = 1;  // the run adds to the caller's x
@@ -2037,8 +2057,7 @@ __global__ void k_add_step(const SolveState *st, const double *__restrict__ p,
 
 // The outer stopping test on the FP64 residual pass's norms.
 static bool outer_converged(const SolveState *h, const sevp_solve_opts *o) {
-  if (o->tol_abs) return sqrt(h->rr64) <= o->tol;
-  return h->bb64 == 0.0 || sqrt(h->rr64 / h->bb64) <= o->tol;
+  return meets_tol(h->rr64, h->bb64, o->tol, o->tol_abs);
 }
 
 // Runs check intervals of an inner iteration until the device state says
@@ -2047,6 +2066,10 @@ static bool outer_converged(const SolveState *h, const sevp_solve_opts *o) {
 // interval is captured once per key (buffers, influence precision, method)
 // and replayed, which needs an even interval so that the buffers return to
 // the same roles.  launches: kernel launches per interval.
+// The intervals queued between polls follow the run's own rate: after each
+// poll, as many as bring the residual to 0.8 of the way to its target in
+// iterations (a poll costs the GPU about 13 us of idling, a launch of a
+// finished run about 1.5 us).
 template <class Interval>
 static int graph_loop(sevp_ctx *ctx, bool graph, const void *const (&key)[5], int check_every,
                       int launches, Interval &&interval, bool pcg_iters = false) {
@@ -2085,19 +2108,29 @@ static int graph_loop(sevp_ctx *ctx, bool graph, const void *const (&key)[5], in
     std::copy(key, key + 5, ctx->inner_graph_key);
   }
   int it0 = 0;  // the run's iterations before this interval (a run starts at 0)
+  int batch = 1;
   for (;;) {
-    if (graph) {
-      SEVP_CUDA_TRY(cudaGraphLaunch(ctx->inner_graph, ctx->stream));
-      ctx->launches += launches;
-    } else {
-      int s = interval(cur);
-      if (s) return s;
+    for (int q = 0; q < batch; ++q) {
+      if (graph) {
+        SEVP_CUDA_TRY(cudaGraphLaunch(ctx->inner_graph, ctx->stream));
+        ctx->launches += launches;
+      } else {
+        int s = interval(cur);
+        if (s) return s;
+      }
     }
     int s = read_state(ctx);
     if (s) return s;
     prof_collect(ctx, pcg_iters ? std::max(ctx->h_st->iter - it0, 0) : -1);
     it0 = ctx->h_st->iter;
     if (ctx->h_st->done) break;
+    batch = 1;
+    const double done_log = log(ctx->h_st->rr / ctx->h_st->bb);
+    const double left_log = log(ctx->h_st->tol2 * ctx->h_st->bb / ctx->h_st->rr);
+    if (pcg_iters && !ctx->prof && it0 > 0 && done_log < -1.0 && left_log < 0.0) {
+      const double left = left_log / done_log * it0;  // iterations at the rate so far
+      batch = std::max(1, std::min(16, (int)(0.8 * left / check_every)));
+    }
   }
   return SEVP_OK;
 }
@@ -2219,6 +2252,20 @@ static int solve_fp64(sevp_ctx *ctx, const double *b, double *x, const sevp_solv
                       sevp_report *rep) {
   const double tol2 = o->tol * o->tol;
   int total = 0, status = SEVP_OK;
+  // the residual pass's norms into the report; true when they meet the
+  // tolerance (st SEVP_OK), st SEVP_NONFINITE when they are not finite
+  auto judge = [&](int &st) {
+    if (!std::isfinite(ctx->h_st->rr64) || !std::isfinite(ctx->h_st->bb64)) {
+      st = SEVP_NONFINITE;
+      return false;
+    }
+    rep->bnorm = sqrt(ctx->h_st->bb64);
+    rep->rel_residual = ctx->h_st->bb64 > 0 ? sqrt(ctx->h_st->rr64 / ctx->h_st->bb64) : 0.0;
+    rep->abs_residual = sqrt(ctx->h_st->rr64);
+    rep->refinements++;
+    st = SEVP_OK;
+    return outer_converged(ctx->h_st, o);
+  };
   for (int restart = 0; restart < 6; ++restart) {
     // the coefficients of the first PCG run are recorded when asked for
     k_state_init<<<1, 1, 0, ctx->stream>>>(ctx->st, tol2, std::max(o->max_iter - total, 0),
@@ -2227,23 +2274,20 @@ static int solve_fp64(sevp_ctx *ctx, const double *b, double *x, const sevp_solv
     // r = b - A x
     int s = launch_residual<double>(ctx, x, nullptr, nullptr, nullptr, b, ctx->r64, 0, tol2);
     if (s) return s;
-    k_state_from_residual<<<1, 1, 0, ctx->stream>>>(ctx->st, tol2, o->tol_abs);
+    k_state_from_residual<<<1, 1, 0, ctx->stream>>>(ctx->st, o->tol, o->tol_abs);
     ctx->launches++;
-    s = read_state(ctx);
-    if (s) return s;
-    if (!std::isfinite(ctx->h_st->rr64) || !std::isfinite(ctx->h_st->bb64)) return SEVP_NONFINITE;
-    double rel = ctx->h_st->bb64 > 0 ? sqrt(ctx->h_st->rr64 / ctx->h_st->bb64) : 0.0;
-    rep->bnorm = sqrt(ctx->h_st->bb64);
-    rep->rel_residual = rel;
-    rep->abs_residual = sqrt(ctx->h_st->rr64);
-    rep->refinements++;
-    if (outer_converged(ctx->h_st, o)) {
-      status = SEVP_OK;
-      break;
-    }
-    if (total >= o->max_iter) {
-      status = SEVP_MAXITER;
-      break;
+    // The first residual rarely meets the tolerance: its run is queued
+    // without waiting for the norms (it ends at once when it does).  The
+    // later ones mostly do and are read first.
+    if (restart > 0 || o->max_iter <= 0) {
+      s = read_state(ctx);
+      if (s) return s;
+      if (judge(status)) break;
+      if (status == SEVP_NONFINITE) return status;
+      if (total >= o->max_iter) {
+        status = SEVP_MAXITER;
+        break;
+      }
     }
     // z = M^{-1} r, rz; then iterate
     s = precondition_pass<double, false, true>(ctx, ctx->r64, nullptr, ctx->z64);
@@ -2252,6 +2296,10 @@ static int solve_fp64(sevp_ctx *ctx, const double *b, double *x, const sevp_solv
     s = pcg_loop<double>(ctx, x, ctx->r64, ctx->z64, ctx->p64[0], ctx->p64[1], ctx->q64,
                          std::max(1, o->check_every), &it);
     if (s) return s;
+    if (restart == 0 && o->max_iter > 0) {
+      if (judge(status)) break;
+      if (status == SEVP_NONFINITE) return status;
+    }
     total += it;
     if (ctx->h_st->x_pend) {
       // iteration k writes its search direction into p64[(k + 1) & 1]
@@ -2333,41 +2381,54 @@ static int solve_mixed(sevp_ctx *ctx, const double *b, double *x, const sevp_sol
     const bool resume = keep && have_dir && !schwarz_on(ctx) && ctx->resume_dev > 0.0;
     if (have_d)
       s = launch_residual<float>(ctx, xa, ctx->d32, last_p, xb, b, ctx->r32, resume ? 2 : 1, inner2,
-                                 outer2, o->tol_abs);
+                                 outer2, o->tol_abs, o->tol);
     else
       s = launch_residual<float>(ctx, xa, nullptr, nullptr, nullptr, b, ctx->r32, 1, inner2, outer2,
-                                 o->tol_abs);
+                                 o->tol_abs, o->tol);
     if (s) return s;
     if (have_d) std::swap(xa, xb);
-    s = read_state(ctx);
-    if (s) return s;
-    if (!std::isfinite(ctx->h_st->rr64) || !std::isfinite(ctx->h_st->bb64)) {
-      status = SEVP_NONFINITE;
-      break;
-    }
-    double rel = ctx->h_st->bb64 > 0 ? sqrt(ctx->h_st->rr64 / ctx->h_st->bb64) : 0.0;
-    rep->bnorm = sqrt(ctx->h_st->bb64);
-    rep->rel_residual = rel;
-    rep->abs_residual = sqrt(ctx->h_st->rr64);
-    rep->refinements++;
-    if (outer_converged(ctx->h_st, o)) {
-      status = SEVP_OK;
-      break;
-    }
-    if (total >= o->max_iter) {
-      status = SEVP_MAXITER;
-      break;
+    // A run whose recursive residual says the tolerance is met by now, and
+    // the Chebyshev iteration, are judged before anything else is queued; the
+    // other runs are queued behind the residual pass (they end at once when
+    // its norms meet the tolerance) and judged with their first poll.
+    const bool read_first = method != SEVP_METHOD_PCG || total >= o->max_iter ||
+                            (have_d && ctx->h_st->rr <= (o->tol_abs ? o->tol * o->tol
+                                                                     : o->tol * o->tol *
+                                                                           ctx->h_st->bb64w));
+    auto judge = [&]() -> bool {  // true: the solve ends with `status`
+      if (!std::isfinite(ctx->h_st->rr64) || !std::isfinite(ctx->h_st->bb64)) {
+        status = SEVP_NONFINITE;
+        return true;
+      }
+      rep->bnorm = sqrt(ctx->h_st->bb64);
+      rep->rel_residual = ctx->h_st->bb64 > 0 ? sqrt(ctx->h_st->rr64 / ctx->h_st->bb64) : 0.0;
+      rep->abs_residual = sqrt(ctx->h_st->rr64);
+      rep->refinements++;
+      if (outer_converged(ctx->h_st, o)) {
+        status = SEVP_OK;
+        return true;
+      }
+      if (total >= o->max_iter) {
+        status = SEVP_MAXITER;
+        return true;
+      }
+      return false;
+    };
+    if (read_first) {
+      s = read_state(ctx);
+      if (s) return s;
+      if (judge()) break;
     }
     // inner solve A d = r32 from d = 0 (a PCG run writes d with its second
     // pass A, or leaves its only step to the residual pass)
     int it = 0;
     if (method == SEVP_METHOD_PCG) {
-      if (!(resume && ctx->h_st->resumed)) {
-        s = precondition_pass<float, false, true>(ctx, ctx->r32, nullptr, ctx->z32);
-        if (s) return s;
-      }
+      // (a resumed run keeps its z: the pass ends at once, SolveState::resumed)
+      s = precondition_pass<float, false, true>(ctx, ctx->r32, nullptr, ctx->z32);
+      if (s) return s;
       s = pcg_loop<float>(ctx, ctx->d32, ctx->r32, ctx->z32, ctx->p32[0], ctx->p32[1], ctx->q32,
                           std::max(1, o->check_every), &it);
+      if (!s && !read_first && judge()) break;
       // iteration k writes its search direction into p32[(k + 1) & 1]; the
       // next loop starts from p32[0]
       if (!s && keep && (it & 1))
