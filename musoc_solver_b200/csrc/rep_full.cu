@@ -13,7 +13,10 @@
 // across matrix elements (MATINV, GEMM); the sequential structure of the
 // method (rows, blocks) is kept.
 #include <algorithm>
+#include <mutex>
 #include <vector>
+
+#include <cooperative_groups.h>
 
 #include "common.cuh"
 #include "dropin.cuh"
@@ -179,6 +182,283 @@ __global__ void __launch_bounds__(1024) k_march_solve(MarchArgs a) {
       X[IXD(ldx, 1, j)] = X[IXD(ldx, a.gi0 - 1, j)];
       X[IXD(ldx, a.gi0, j)] = X[IXD(ldx, 2, j)];
     }
+  }
+}
+
+// The marching solve on a cluster of kMarchCtas CTAs, for grids whose blocks'
+// rows fit their shared memory.
+//
+// k_march_solve is one CTA that reads each influence matrix (m2 x m2) for one
+// serial mat-vec: 44 of them at 180 x 90 with 15 blocks, each 259 KB through
+// one SM in dependent batches, and every marched row goes through global
+// memory; 655 us.  Here the mat-vecs' output columns are split over the
+// cluster: a CTA copies its columns of the next two matrices to shared memory
+// while the rows march (cp.async), sums its outputs in the reference's serial
+// order from there (two instructions' latency per term), and writes them to
+// every CTA of the cluster.  All CTAs march all rows themselves, one column
+// per thread, on rows in shared memory with the coefficients two rows ahead
+// in registers, so the mat-vec results are all that is exchanged.  CTA 0
+// writes the outputs; the other CTAs read of X only input rows that it has
+// not written yet (the guess rows, in the forward sweep).
+// The arithmetic of every value is that of k_march_solve, so the results are
+// bit-identical.
+constexpr int kMarchCtas = 8;
+constexpr int kMarchMaxCols = 512;  // one thread per column
+
+struct MarchCoef {
+  float ax, ay, bb, cx, cy, f;
+  double e;  // forward: row j + 2's ghost cell (closed grids); backward: X(., j + 2)
+};
+
+// Doubles of shared memory: saved rows (ie - 1, ie, guess) per block, two
+// matrix slices, three rows, the mat-vec input and two outputs.
+__host__ __device__ inline size_t march_smem_doubles(int m2, int nblk, int nper) {
+  return (size_t)3 * nblk * m2 + (size_t)2 * nper * (m2 | 1) + (size_t)3 * (m2 + 2) +
+         (size_t)3 * m2;
+}
+
+__global__ void __cluster_dims__(kMarchCtas, 1, 1) __launch_bounds__(kMarchMaxCols, 1)
+    k_march_cluster(MarchArgs a, int nper) {
+  namespace cg = cooperative_groups;
+  cg::cluster_group cl = cg::this_cluster();
+  extern __shared__ __align__(16) double msm[];
+  const int rank = (int)cl.block_rank();
+  const int m2 = a.m2, nblk = a.nblk, ldr = m2 | 1, ld = m2 + 2;
+  const int tid = threadIdx.x, i = tid + 1, nt = blockDim.x;
+  const bool act = tid < m2, lead = rank == 0, per = a.periodic != 0;
+  const size_t msz = (size_t)m2 * m2;
+  double *SA = msm, *D0 = SA + (size_t)nblk * m2, *G = D0 + (size_t)nblk * m2;
+  double *Rb = G + (size_t)nblk * m2, *rows = Rb + (size_t)2 * nper * ldr;
+  double *vin = rows + 3 * ld, *vout = vin + m2;
+  const int n0 = rank * nper, cnt = max(0, min(nper, m2 - n0));
+  const int last = a.ie[nblk - 1], crows = last - 1;
+
+  // ---- the mat-vecs, in the order of the sweeps
+  auto matrix = [&](int q) -> const double * {
+    if (q < nblk - 1) return a.rinv1 + (size_t)q * msz;
+    const int p = q - (nblk - 1), nb = nblk - p / 2;
+    return (p & 1) ? a.rinv1 + (size_t)(nb - 2) * msz : a.rinv + (size_t)(nb - 1) * msz;
+  };
+  const int nq = 3 * nblk - 2;
+  auto prefetch = [&](int q) {
+    if (q < nq) {
+      const double *R = matrix(q) + (size_t)n0 * m2;
+      double *dst = Rb + (size_t)(q & 1) * nper * ldr;
+      for (int c = tid >> 5; c < cnt; c += nt >> 5)
+        for (int k = tid & 31; k < m2; k += 32) {
+          const unsigned d = (unsigned)__cvta_generic_to_shared(dst + (size_t)c * ldr + k);
+          asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(d),
+                       "l"(R + (size_t)c * m2 + k)
+                       : "memory");
+        }
+    }
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+  };
+  int q = 0;
+  prefetch(0);
+  prefetch(1);
+  cl.sync();  // every CTA runs before any writes to another's shared memory
+  // out(n) = sum_k vin(k) R(k, n) for all n, on every CTA (vin is written by
+  // the caller's threads just before)
+  auto matvec = [&]() -> const double * {
+    asm volatile("cp.async.wait_group 1;\n" ::: "memory");
+    __syncthreads();
+    double *out = vout + (size_t)(q & 1) * m2;
+    if (tid < cnt) {
+      const double *col = Rb + (size_t)(q & 1) * nper * ldr + (size_t)tid * ldr;
+      double s = 0.0;
+      int k = 0;
+      for (; k + kVecmatBatch <= m2; k += kVecmatBatch) {
+        double c[kVecmatBatch], v[kVecmatBatch];
+#pragma unroll
+        for (int u = 0; u < kVecmatBatch; ++u) c[u] = col[k + u], v[u] = vin[k + u];
+#pragma unroll
+        for (int u = 0; u < kVecmatBatch; ++u) s = add(s, mul(v[u], c[u]));
+      }
+      for (; k < m2; ++k) s = add(s, mul(vin[k], col[k]));
+      for (int r = 0; r < kMarchCtas; ++r) cl.map_shared_rank(out, r)[n0 + tid] = s;
+    }
+    // the other output buffer is not written before every CTA has passed the
+    // next barrier, so this one stays whole until all have read it
+    cl.sync();
+    prefetch(q + 2);
+    ++q;
+    return out;
+  };
+  auto coef = [&](int j, bool back) {
+    MarchCoef c{};
+    if (!act || j < 1 || j > crows) return c;
+    const size_t o = IXD(a.ldc, i, j);
+    c.ax = __ldg(a.ax + o), c.ay = __ldg(a.ay + o), c.bb = __ldg(a.bb + o);
+    c.cx = __ldg(a.cx + o), c.cy = __ldg(a.cy + o);
+    if (!back) {
+      c.f = __ldg(a.f + IXD(a.ldf, i, j));
+      if (!per && (tid == 0 || tid == m2 - 1))
+        c.e = a.x[IXD(a.ldx, tid == 0 ? 1 : m2 + 2, j + 2)];
+    } else if (lead) {
+      c.e = a.x[IXD(a.ldx, i + 1, j + 2)];
+    }
+    return c;
+  };
+  // the five-point terms of a row, in march_val's and resid_val's order
+  auto terms = [&](const MarchCoef &c, double f, double w, double s, double m, double e) {
+    double t = sub(f, mul((double)c.ax, w));
+    t = sub(t, mul((double)c.ay, s));
+    t = sub(t, mul((double)c.bb, m));
+    return sub(t, mul((double)c.cx, e));
+  };
+  // a value into a row in shared memory, with the row's ghost cells: periodic
+  // copies, or gh (the cell next to the first and last column)
+  auto put = [&](double *row, double v, double gh) {
+    if (!act) return;
+    row[i] = v;
+    if (tid == m2 - 1) row[per ? 0 : m2 + 1] = per ? v : gh;
+    if (tid == 0) row[per ? m2 + 1 : 0] = per ? v : gh;
+  };
+  auto xval = [&](int j) { return act ? a.x[IXD(a.ldx, i + 1, j)] : 0.0; };
+  auto xghost = [&](int j) {
+    return (!per && act && (tid == 0 || tid == m2 - 1))
+               ? a.x[IXD(a.ldx, tid == 0 ? 1 : m2 + 2, j)]
+               : 0.0;
+  };
+  double *S = rows, *C = rows + ld, *N = rows + 2 * ld;
+  auto rotate = [&]() {
+    double *t = S;
+    S = C, C = N, N = t;
+  };
+
+  // ---- forward sweep
+  put(S, xval(1), xghost(1));
+  put(C, xval(2), xghost(2));
+  MarchCoef p0 = coef(1, false), p1 = coef(2, false);
+  int js = 1;
+  double north = 0.0;
+  __syncthreads();
+  for (int nb = 1; nb <= nblk; ++nb) {
+    const int ie = a.ie[nb - 1], jf = ie - 2;
+    // the row above the block: its guess row above, or the north boundary
+    north = xval(ie + 1);
+    const double north_gh = xghost(ie + 1);
+    if (act) G[(size_t)(nb - 1) * m2 + tid] = C[i];
+    for (int j = js; j <= jf; ++j) {
+      const MarchCoef c = p0;
+      p0 = p1;
+      p1 = coef(j + 2, false);
+      if (act) {
+        const double v = dvd(terms(c, (double)c.f, C[i - 1], S[i], C[i], C[i + 1]), (double)c.cy);
+        put(N, v, c.e);
+        if (lead) a.x[IXD(a.ldx, i + 1, j + 2)] = v;
+      }
+      __syncthreads();
+      rotate();
+    }
+    if (act) {
+      SA[(size_t)(nb - 1) * m2 + tid] = S[i];
+      D0[(size_t)(nb - 1) * m2 + tid] = C[i];
+    }
+    if (nb != nblk) {
+      const MarchCoef c = p0;
+      p0 = p1;
+      p1 = coef(ie + 1, false);
+      if (act) {
+        const double t = terms(c, (double)c.f, C[i - 1], S[i], C[i], C[i + 1]);
+        vin[tid] = sub(t, mul((double)c.cy, north));
+      }
+      const double *o = matvec();
+      if (act) {
+        const double d = C[i];
+        if (lead) a.dum0[IXD(m2, i, nb)] = d;
+        put(N, sub(d, o[tid]), 0.0);  // the corrected row: the next block's south row
+        put(S, north, north_gh);      // its guess row
+      }
+      double *t = S;  // (S, C, N) = (corrected, guess, free)
+      S = N, N = C, C = t;
+      __syncthreads();
+    }
+    js = ie;
+  }
+  // ---- backward sweep
+  MarchCoef rc = coef(last - 1, false);
+  double res = 0.0;
+  const double *o = nullptr;
+  for (int nb = nblk; nb >= 1; --nb) {
+    const int ie = a.ie[nb - 1], jf = ie - 2;
+    js = nb != 1 ? a.ie[nb - 2] : 1;
+    const double *d0 = D0 + (size_t)(nb - 1) * m2;
+    if (lead)
+      for (int j = js; j <= ie; ++j)
+        for (int k = 1 + tid; k <= a.hzero; k += nt) a.h[IXD(a.ldh, k, j)] = 0.0;
+    if (act) {
+      double w, e;
+      if (per) {
+        w = d0[tid > 0 ? tid - 1 : m2 - 1];
+        e = d0[tid < m2 - 1 ? tid + 1 : 0];
+      } else {
+        w = tid > 0 ? d0[tid - 1] : a.x[IXD(a.ldx, 1, ie)];
+        e = tid < m2 - 1 ? d0[tid + 1] : a.x[IXD(a.ldx, m2 + 2, ie)];
+      }
+      const double t = terms(rc, (double)rc.f, w, SA[(size_t)(nb - 1) * m2 + tid], d0[tid], e);
+      res = sub(t, mul((double)rc.cy, north));
+      vin[tid] = res;
+    }
+    const float cy_s = nb != 1 && act ? __ldg(a.cy + IXD(a.ldc, i, js - 1)) : 0.f;
+    p0 = coef(js, true), p1 = coef(js + 1, true);
+    o = matvec();
+    const double v = act ? o[tid] : 0.0;
+    if (act) {
+      north = add(G[(size_t)(nb - 1) * m2 + tid], v);
+      put(C, v, 0.0);
+      S[i] = 0.0;
+      if (lead) {
+        a.h[IXD(a.ldh, i + 1, js + 1)] = v;
+        a.x[IXD(a.ldx, i + 1, js + 1)] = north;
+        if (per && tid == m2 - 1) a.h[IXD(a.ldh, 1, js + 1)] = v;
+        if (per && tid == 0) a.h[IXD(a.ldh, a.gi0, js + 1)] = v;
+      }
+    }
+    if (nb != 1) {
+      if (act) vin[tid] = mul(v, (double)cy_s);
+      o = matvec();
+      if (act) {
+        const double hv = o[tid];
+        S[i] = hv;
+        if (lead) {
+          a.h[IXD(a.ldh, i + 1, js)] = hv;
+          if (per && tid == m2 - 1) a.h[IXD(a.ldh, 1, js)] = hv;
+          if (per && tid == 0) a.h[IXD(a.ldh, a.gi0, js)] = hv;
+        }
+      }
+      rc = coef(js - 1, false);
+    }
+    __syncthreads();
+    for (int j = js; j <= jf; ++j) {
+      const MarchCoef c = p0;
+      p0 = p1;
+      p1 = coef(j + 2, true);
+      if (act) {
+        const double hv = dvd(terms(c, 0.0, C[i - 1], S[i], C[i], C[i + 1]), (double)c.cy);
+        put(N, hv, 0.0);
+        if (lead) {
+          a.h[IXD(a.ldh, i + 1, j + 2)] = hv;
+          a.x[IXD(a.ldx, i + 1, j + 2)] = add(c.e, hv);
+          if (per && j < jf) {
+            if (tid == m2 - 1) a.h[IXD(a.ldh, 1, j + 2)] = hv;
+            if (tid == 0) a.h[IXD(a.ldh, a.gi0, j + 2)] = hv;
+          }
+        }
+      }
+      __syncthreads();
+      rotate();
+    }
+  }
+  if (lead) {
+    if (act) a.dum1[tid] = res, a.dum2[tid] = o[tid];
+    __syncthreads();
+    if (per)
+      for (int j = 2 + tid; j <= last; j += nt) {
+        a.x[IXD(a.ldx, 1, j)] = a.x[IXD(a.ldx, a.gi0 - 1, j)];
+        a.x[IXD(a.ldx, a.gi0, j)] = a.x[IXD(a.ldx, 2, j)];
+      }
   }
 }
 
@@ -406,6 +686,23 @@ __global__ void k_periodic_cols(double *x, int i2, int j2) {
 
 // ------------------------------------------------------------ host side
 int dev_march_solve(const MarchArgs &a, cudaStream_t st) {
+  // the cluster where a column has a thread, the blocks' rows fit its shared
+  // memory, and H's zeroed columns cover the ghosts (the reference's shapes)
+  const int nper = ceil_div(a.m2, kMarchCtas);
+  const size_t smem = march_smem_doubles(a.m2, a.nblk, nper) * sizeof(double);
+  if (a.m2 >= 2 && a.m2 <= kMarchMaxCols && a.hzero >= a.m2 + 2 &&
+      (!a.periodic || a.gi0 == a.m2 + 2) && smem <= (size_t)220 * 1024) {
+    static std::once_flag once;
+    static cudaError_t err = cudaSuccess;
+    std::call_once(once, [] {
+      err = cudaFuncSetAttribute(k_march_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 220 * 1024);
+    });
+    SEVP_CUDA_TRY(err);
+    k_march_cluster<<<kMarchCtas, ceil_div(a.m2, 32) * 32, smem, st>>>(a, nper);
+    SEVP_CUDA_TRY(cudaGetLastError());
+    return SEVP_OK;
+  }
   int threads = std::min(1024, std::max(32, ((a.m2 + 31) / 32) * 32));
   k_march_solve<<<1, threads, 0, st>>>(a);
   SEVP_CUDA_TRY(cudaGetLastError());

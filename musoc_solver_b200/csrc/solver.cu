@@ -69,6 +69,8 @@ __global__ void __launch_bounds__(kStencilThreads, SEVP_STENCIL_MINB)
   using T = typename Op::T;
   // rows per step: all their loads are issued together
   constexpr int U = SEVP_STENCIL_UNROLL > 0 ? SEVP_STENCIL_UNROLL : (sizeof(T) == 4 ? 4 : 2);
+  pdl_trigger();
+  pdl_wait();
   if (Op::kUsesState && st->done) return;
   op.prepare(st);
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -1131,7 +1133,11 @@ extern "C" const char *sevp_status_string(int s) {
 
 // Rows per CTA of the stencil kernels, chosen once per context: a CTA loads
 // rpw + 2 rows, and the grid runs in ceil(CTAs / slots) waves, so pick the
-// rpw in [8, 32] that minimises waves x (rpw + 2) (ties: more rows).
+// rpw in [2, 32] that minimises waves x (rpw + 2) (ties: more rows).  Small
+// grids fit one wave at any rpw and take 2 rows: their passes are a CTA's
+// latency (residual pass at 180 x 90: 15.6 us with 8 rows).  The partial-sum
+// buffer has room for five sums per CTA (kStencilSums).
+constexpr int kStencilSums = 5;
 static int stencil_rpw(sevp_ctx *ctx) {
   if (ctx->stencil_rpw > 0) return ctx->stencil_rpw;
   int dev = 0, sms = 148;
@@ -1141,8 +1147,9 @@ static int stencil_rpw(sevp_ctx *ctx) {
   const long long gx = ceil_div(ceil_div(ctx->nx, kStencilCols), kStencilThreads / 32);
   int best = 8;
   long long best_cost = -1;
-  for (int rpw = 8; rpw <= 32; ++rpw) {
+  for (int rpw = 2; rpw <= 32; ++rpw) {
     const long long ctas = gx * ceil_div(ctx->ny, rpw);
+    if (rpw < 8 && ctas * kStencilSums > (long long)ctx->partials_n) continue;
     const long long cost = ((ctas + slots - 1) / slots) * (rpw + 2);
     if (best_cost < 0 || cost <= best_cost) best = rpw, best_cost = cost;
   }
@@ -1164,14 +1171,10 @@ static int launch_stencil_c(sevp_ctx *ctx, const Op &op, int ticket_slot, const 
   dim3 grid = stencil_grid(ctx, rpw);
   GridDims gd{ctx->nx, ctx->ny, ctx->periodic};
   ProfScope ps(ctx, 1);
-  if (sym)
-    k_stencil<Op, true><<<grid, kStencilThreads, 0, ctx->stream>>>(
-        gd, c, op, rpw, ctx->partials, ctx->tickets + ticket_slot, ctx->st);
-  else
-    k_stencil<Op, false><<<grid, kStencilThreads, 0, ctx->stream>>>(
-        gd, c, op, rpw, ctx->partials, ctx->tickets + ticket_slot, ctx->st);
   ctx->launches++;
-  SEVP_CUDA_TRY(cudaGetLastError());
+  SEVP_CUDA_TRY(launch_overlapped(sym ? k_stencil<Op, true> : k_stencil<Op, false>, grid,
+                                  kStencilThreads, 0, ctx->stream, true, gd, c, op, rpw,
+                                  ctx->partials, ctx->tickets + ticket_slot, ctx->st));
   return SEVP_OK;
 }
 template <class Op>
