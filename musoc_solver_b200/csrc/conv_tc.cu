@@ -268,7 +268,7 @@ __global__ void __launch_bounds__(kTcThreads)
 // channels-contiguous (NHWC) in memory, so the staging transposes them into
 // the K-major no-swizzle core-matrix layout of k_conv3x3_tc: a thread loads
 // 8 channels of two neighbouring pixels (two 16-byte loads) and writes eight
-// 4-byte (k, k+1) pairs, one per row.  Thread 0 issues the K = 16 MMAs of a
+// 4-byte (k, k+1) pairs, one per row (store_k_pairs).  Thread 0 issues the K = 16 MMAs of a
 // step and commits them to the stage's mbarrier; with kWgStages stages a
 // stage is refilled while the MMAs of the two before it run.  The FP32 tile
 // in TMEM is added to dW with atomics (the pixel chunks of a tap are spread
@@ -276,15 +276,30 @@ __global__ void __launch_bounds__(kTcThreads)
 constexpr int kWgStages = 3;
 constexpr int kWgK = 64;  // pixels per step
 
-__device__ __forceinline__ void store_k_pairs(unsigned char *base, int grp, int k, const uint4 &v0,
-                                              const uint4 &v1) {
-  // rows 8 grp .. 8 grp + 7, K elements k and k + 1 (k even)
-  const uint16_t *a = reinterpret_cast<const uint16_t *>(&v0);
-  const uint16_t *b = reinterpret_cast<const uint16_t *>(&v1);
+// Writes rows 8 grp .. 8 grp + 7, K elements k and k + 1 (k even), one 4-byte
+// word per row.  The word of row j lies in bank 4 j + (k / 2) mod 4 for every
+// grp and every multiple of 8 in k, so lanes that share k / 2 mod 4 write
+// their rows in orders rotated by rot (0..7, different for those lanes):
+// eight conflict-free stores instead of eight 8- to 32-way conflicts.
+__device__ __forceinline__ void store_k_pairs(unsigned char *base, int grp, int k, int rot,
+                                              const uint4 &v0, const uint4 &v1) {
+  const uint32_t p[4] = {v0.x, v0.y, v0.z, v0.w}, n[4] = {v1.x, v1.y, v1.z, v1.w};
+  uint32_t w[8], u[8];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    w[2 * j] = __byte_perm(p[j], n[j], 0x5410);
+    w[2 * j + 1] = __byte_perm(p[j], n[j], 0x7632);
+  }
+#pragma unroll
+  for (int j = 0; j < 8; ++j) u[j] = (rot & 1) ? w[(j + 1) & 7] : w[j];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) w[j] = (rot & 2) ? u[(j + 2) & 7] : u[j];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) u[j] = (rot & 4) ? w[(j + 4) & 7] : w[j];
   unsigned char *core = base + (k >> 3) * 128 + grp * (kWgK / 8 * 128) + (k & 7) * 2;
 #pragma unroll
   for (int j = 0; j < 8; ++j)
-    *reinterpret_cast<uint32_t *>(core + j * 16) = (uint32_t)a[j] | ((uint32_t)b[j] << 16);
+    *reinterpret_cast<uint32_t *>(core + ((j + rot) & 7) * 16) = u[j];
 }
 
 __global__ void __launch_bounds__(kTcThreads)
@@ -328,37 +343,62 @@ __global__ void __launch_bounds__(kTcThreads)
   tc_fence_after();
   const uint32_t tmem = s_tmem;
 
+  // A warp copies 8-channel groups of pixel pairs: lane bits 0-1 pick the pair
+  // (of four with different banks), the others the group, so that a load
+  // covers up to 128 contiguous bytes per pixel, and then further pairs.
+  const int rot = lane >> 2;
+  const uint4 zero = make_uint4(0, 0, 0, 0);
+  auto groups = [](int n) { return n >= 8 ? 8 : (n >= 4 ? 4 : 2); };  // n >= 2
   auto stage = [&](int s) {
     unsigned char *a_p = sm + (s % kWgStages) * stage_bytes;
     unsigned char *b_p = a_p + a_bytes;
     const long long k0 = pb + (long long)s * kWgK;
-    const uint4 zero = make_uint4(0, 0, 0, 0);
     const int mg = mrows / 8, ng = cin / 8;
-    for (int e = tid; e < (kWgK / 2) * mg; e += kTcThreads) {
-      const int kp = e / mg, grp = e - kp * mg, k = 2 * kp;
-      const long long p = k0 + k;
-      const uint4 v0 = p < pe ? *reinterpret_cast<const uint4 *>(g + p * cout + co0 + grp * 8) : zero;
-      const uint4 v1 =
-          p + 1 < pe ? *reinterpret_cast<const uint4 *>(g + (p + 1) * cout + co0 + grp * 8) : zero;
-      store_k_pairs(a_p, grp, k, v0, v1);
-    }
-    for (int e = tid; e < (kWgK / 2) * ng; e += kTcThreads) {
-      const int kp = e / ng, grp = e - kp * ng, k = 2 * kp;
-      uint4 v[2];
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const long long p = k0 + k + h;
-        v[h] = zero;
-        if (p < pe) {
-          const long long img = p / HW;
-          const int rem = (int)(p - img * HW);
-          const int yy = rem / W + dy, xx = rem - (rem / W) * W + dx;
-          if (yy >= 0 && yy < H && xx >= 0 && xx < W)
-            v[h] = *reinterpret_cast<const uint4 *>(
-                x + ((img * H + yy) * W + xx) * x_ld + x_off + grp * 8);
+    {
+      const int gw = groups(mg), pairs = 32 / gw;  // pixel pairs per warp copy
+      const int kl = (lane & 3) + 4 * (rot / gw), gl = rot % gw;
+      for (int kp = warp * pairs + kl; kp < kWgK / 2; kp += 4 * pairs) {
+        const long long p = k0 + 2 * kp;
+        const bf16 *src = g + p * cout + co0;
+        for (int grp = gl; grp < mg; grp += gw) {
+          const uint4 v0 = p < pe ? *reinterpret_cast<const uint4 *>(src + grp * 8) : zero;
+          const uint4 v1 =
+              p + 1 < pe ? *reinterpret_cast<const uint4 *>(src + cout + grp * 8) : zero;
+          store_k_pairs(a_p, grp, 2 * kp, rot, v0, v1);
         }
       }
-      store_k_pairs(b_p, grp, k, v[0], v[1]);
+    }
+    {
+      const int gw = groups(ng), pairs = 32 / gw;
+      const int kl = (lane & 3) + 4 * (rot / gw), gl = rot % gw;
+      for (int kp = warp * pairs + kl; kp < kWgK / 2; kp += 4 * pairs) {
+        const bf16 *src[2] = {nullptr, nullptr};
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const long long p = k0 + 2 * kp + h;
+          if (p >= pe) continue;
+          long long img;
+          int yy, xx;
+          if (P <= 0xffffffffLL) {  // 32-bit divisions
+            const unsigned row = (unsigned)p / (unsigned)W, im = row / (unsigned)H;
+            xx = (int)((unsigned)p - row * (unsigned)W) + dx;
+            yy = (int)(row - im * (unsigned)H) + dy;
+            img = im;
+          } else {
+            img = p / HW;
+            const long long rem = p - img * HW;
+            yy = (int)(rem / W) + dy;
+            xx = (int)(rem % W) + dx;
+          }
+          if (yy >= 0 && yy < H && xx >= 0 && xx < W)
+            src[h] = x + ((img * H + yy) * W + xx) * x_ld + x_off;
+        }
+        for (int grp = gl; grp < ng; grp += gw) {
+          const uint4 v0 = src[0] ? *reinterpret_cast<const uint4 *>(src[0] + grp * 8) : zero;
+          const uint4 v1 = src[1] ? *reinterpret_cast<const uint4 *>(src[1] + grp * 8) : zero;
+          store_k_pairs(b_p, grp, 2 * kp, rot, v0, v1);
+        }
+      }
     }
   };
 

@@ -221,6 +221,40 @@ __global__ void k_bias_grad(const bf16 *dy, int dy_ld, int dy_off, int cout, con
   atomicAdd(&db[co], s);
 }
 
+// Sums 8 channels per thread over the CTA's threads with the same channel
+// group (tid % C8; C8 a power of two, at most the CTA's 256 threads) and adds
+// the sums of group q to out[8 q .. 8 q + 7], one atomic per channel and CTA.
+__device__ __forceinline__ void add_group_sums(float (&s)[8], int C8, float *sh, float *out) {
+  const int tid = threadIdx.x;
+#pragma unroll
+  for (int k = 0; k < 8; ++k) sh[k * 256 + tid] = s[k];
+  __syncthreads();
+  for (int e = tid; e < 8 * C8; e += 256) {
+    const int q = e >> 3, k = e & 7;
+    float t = 0.f;
+    for (int r = q; r < 256; r += C8) t += sh[k * 256 + r];
+    atomicAdd(out + e, t);
+  }
+}
+
+// k_bias_grad for packed, unmasked gradients of 8 C8 channels (C8 a power of
+// two): 8 channels per thread in 16-byte loads, every thread busy (with one
+// channel per thread a 32-channel layer kept an eighth of the CTA).
+__global__ void __launch_bounds__(256)
+    k_bias_grad8(const bf16 *__restrict__ dy, int C8, float *db, long long P) {
+  __shared__ float sh[8 * 256];
+  float s[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+  const long long n = P * C8;  // a thread's channel group is the same in every round
+  for (long long e = (long long)blockIdx.x * 256 + threadIdx.x; e < n;
+       e += (long long)gridDim.x * 256) {
+    const uint4 v = *reinterpret_cast<const uint4 *>(dy + e * 8);
+    const bf16 *b = reinterpret_cast<const bf16 *>(&v);
+#pragma unroll
+    for (int k = 0; k < 8; ++k) s[k] += __bfloat162float(b[k]);
+  }
+  add_group_sums(s, C8, sh, db);
+}
+
 // transposed, tap-mirrored copy for the data gradient: wt[tap][co][ci] = w[tap][ci][co]
 __global__ void k_weight_transpose(const bf16 *w, bf16 *wt, int cin, int cout) {
   const size_t n = (size_t)9 * cin * cout;
@@ -437,6 +471,40 @@ __global__ void k_head_bwd(const bf16 *x, int x_ld, int x_off, int C, const floa
   if (threadIdx.x == 0) atomicAdd(db, sw[C]);
 }
 
+// k_head_bwd for 8 C8 channels (C8 a power of two, at most 256 threads) in
+// 16-byte groups: the channel sums stay in registers until the end (a shared-
+// memory atomic per pixel and channel serialised the CTA: 105 us for 184 x 360
+// pixels of 32 channels).
+__global__ void __launch_bounds__(256)
+    k_head_bwd8(const bf16 *__restrict__ x, int x_ld, int x_off, int C8,
+                const float *__restrict__ w, const float *__restrict__ dy, bf16 *dx, int dx_ld,
+                int dx_off, float *dw, float *db, long long P) {
+  __shared__ float sh[8 * 256];
+  const int tid = threadIdx.x, q = tid % C8;
+  float wv[8], s[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f}, sg = 0.f;
+#pragma unroll
+  for (int k = 0; k < 8; ++k) wv[k] = w[8 * q + k];
+  const int per = 256 / C8;  // pixels per CTA and round
+  for (long long p = (long long)blockIdx.x * per + tid / C8; p < P;
+       p += (long long)gridDim.x * per) {
+    const float g = dy[p];
+    const uint4 v = *reinterpret_cast<const uint4 *>(x + p * x_ld + x_off + 8 * q);
+    const bf16 *b = reinterpret_cast<const bf16 *>(&v);
+    __align__(16) bf16 o[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      o[k] = __float2bfloat16(g * wv[k]);
+      s[k] += g * __bfloat162float(b[k]);
+    }
+    *reinterpret_cast<uint4 *>(dx + p * dx_ld + dx_off + 8 * q) =
+        *reinterpret_cast<const uint4 *>(o);
+    if (q == 0) sg += g;
+  }
+  add_group_sums(s, C8, sh, dw);
+  for (int o = 16; o > 0; o >>= 1) sg += __shfl_xor_sync(0xffffffffu, sg, o);
+  if ((tid & 31) == 0 && sg != 0.f) atomicAdd(db, sg);
+}
+
 // loss = mean (y - t)^2 over valid pixels; dy = 2 (y - t) / n
 __global__ void k_mse(const float *y, const float *t, const float *valid, float *dy, float *loss,
                       long long P, float inv_n) {
@@ -583,8 +651,16 @@ int sevp_nn_conv3x3_backward_tc(const void *x, int x_ld, int x_off, int cin, con
   int s = sevp_nn_conv3x3_wgrad_tc(x, x_ld, x_off, cin, scratch, cout, dw, B, H, W, stream);
   if (s) return s;
   if (db) {
-    dim3 g2(256, (unsigned)((cout + 255) / 256));
-    k_bias_grad<<<g2, 256, 0, st>>>((const bf16 *)scratch, cout, 0, cout, nullptr, 0, 0, db, P);
+    const int c8 = cout / 8;
+    if ((c8 & (c8 - 1)) == 0) {
+      // about eight rounds per thread, so that a CTA's sums and atomics stay few
+      const long long ctas = (P * c8 + 256 * 8 - 1) / (256 * 8);
+      k_bias_grad8<<<(unsigned)std::min<long long>(std::max<long long>(ctas, 1), 148), 256, 0, st>>>(
+          (const bf16 *)scratch, c8, db, P);
+    } else {
+      dim3 g2(256, (unsigned)((cout + 255) / 256));
+      k_bias_grad<<<g2, 256, 0, st>>>((const bf16 *)scratch, cout, 0, cout, nullptr, 0, 0, db, P);
+    }
     SEVP_CUDA_TRY(cudaGetLastError());
   }
   if (!dx) return SEVP_OK;
@@ -652,8 +728,17 @@ int sevp_nn_head(const void *x, int x_ld, int x_off, int C, const float *w, cons
       k_head_fwd<<<ew_grid(P), 256, 0, st>>>((const bf16 *)x, x_ld, x_off, C, w, b, y, P);
   } else {
     if (!dy || !dx || !dw || !db) return SEVP_BAD_ARG;
-    k_head_bwd<<<ew_grid(P), 256, 0, st>>>((const bf16 *)x, x_ld, x_off, C, w, dy, (bf16 *)dx, dx_ld,
-                                           dx_off, dw, db, P);
+    const int c8 = C / 8;
+    if (C % 8 == 0 && (c8 & (c8 - 1)) == 0 && c8 <= 32 && x_ld % 8 == 0 && x_off % 8 == 0 &&
+        dx_ld % 8 == 0 && dx_off % 8 == 0 && (((uintptr_t)x | (uintptr_t)dx) & 15) == 0) {
+      const long long ctas = (P * c8 + 256 * 4 - 1) / (256 * 4);
+      k_head_bwd8<<<(unsigned)std::min<long long>(std::max<long long>(ctas, 1), 2 * 148), 256, 0,
+                    st>>>((const bf16 *)x, x_ld, x_off, c8, w, dy, (bf16 *)dx, dx_ld, dx_off, dw,
+                          db, P);
+    } else {
+      k_head_bwd<<<ew_grid(P), 256, 0, st>>>((const bf16 *)x, x_ld, x_off, C, w, dy, (bf16 *)dx, dx_ld,
+                                             dx_off, dw, db, P);
+    }
   }
   SEVP_CUDA_TRY(cudaGetLastError());
   return SEVP_OK;
