@@ -198,7 +198,12 @@ struct OpPassA {
     if (step) x[idx] = fma_rn(alpha, pold[idx], x_init ? x[idx] : V(0));
     acc[0] += (double)vc * (double)av;
   }
-  __device__ void operator()(double (&s)[NV]) { PassAFin{st}(s); }
+  PassAFin fin;
+  __device__ void load() {
+    fin.st = st;
+    fin.load();
+  }
+  __device__ void operator()(double (&s)[NV]) { fin(s); }
 };
 
 // The outer stopping test on an FP64 residual pass's norms ||b - A x||^2 and

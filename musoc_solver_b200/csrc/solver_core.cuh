@@ -78,8 +78,21 @@ __device__ __forceinline__ T stencil5(float cb, T vb, float cw, T vw, float cc, 
 }
 
 // ------------------------------------------------- reductions / finisher
+// A finisher may have load(): what it needs of the state, read by every CTA's
+// first thread while its sums travel (the state does not change before the
+// last CTA's finisher), so that the finisher itself waits for no memory.
+template <class Fin>
+__device__ __forceinline__ auto fin_load(Fin &fin, int) -> decltype(fin.load(), void()) {
+  fin.load();
+}
+template <class Fin>
+__device__ __forceinline__ void fin_load(Fin &, long) {}
+
 // Writes this CTA's NV partial sums, and lets the last CTA to arrive sum all
-// partials in block order and call fin(sums) once.
+// partials in block order and call fin(sums) once.  On a small grid this is
+// most of a pass (a store and its fence cost 0.4 us, a dependent read of the
+// state as much), so the finisher's reads come with the fence and nothing is
+// fenced at the end (the kernel's end makes the writes visible).
 template <int NV, class Fin>
 __device__ __forceinline__ void reduce_and_finish(double (&v)[NV], double *partials,
                                                   unsigned *ticket, Fin &fin) {
@@ -91,6 +104,7 @@ __device__ __forceinline__ void reduce_and_finish(double (&v)[NV], double *parti
   if (threadIdx.x == 0) {
 #pragma unroll
     for (int k = 0; k < NV; ++k) partials[(size_t)bid * NV + k] = v[k];
+    fin_load(fin, 0);
     __threadfence();
     unsigned t = atomicAdd(ticket, 1u);
     s_last = (t == (unsigned)nblk - 1u);
@@ -109,7 +123,6 @@ __device__ __forceinline__ void reduce_and_finish(double (&v)[NV], double *parti
     if (threadIdx.x == 0) {
       fin(acc);
       *ticket = 0u;
-      __threadfence();
     }
   }
 }
@@ -227,9 +240,16 @@ __device__ __forceinline__ double march_rcp(double a) {
 // Finishes a PCG iteration after pass B: r.z and r.r are complete.
 struct TileFin {
   SolveState *st;
+  double beta, rz_old, limit, *hist;
+  int iter, max_iter, keep_dir, hist_cap;
+  __device__ void load() {
+    beta = st->beta, rz_old = st->rz, limit = st->tol2 * st->bb;
+    iter = st->iter, max_iter = st->max_iter, keep_dir = st->keep_dir;
+    hist = st->hist, hist_cap = st->hist_cap;
+  }
   __device__ void operator()(double (&s)[2]) {
     double rz = s[0], rr = s[1];
-    int first = (st->beta == 0.0 && st->iter == 0 && !st->keep_dir);
+    int first = (beta == 0.0 && iter == 0 && !keep_dir);
     st->keep_dir = 0;
     st->rr = rr;
     st->rz_next = rz;
@@ -241,12 +261,12 @@ struct TileFin {
     // a finished run keeps the previous r.z: a continuation after a
     // residual replacement takes beta = (new r.z) / (that r.z), the step
     // this run would have taken next
-    if (rr <= st->tol2 * st->bb) {
+    if (rr <= limit) {
       st->done = 1;
       st->status = SEVP_OK;
       return;
     }
-    if (st->iter >= st->max_iter) {
+    if (iter >= max_iter) {
       st->done = 1;
       st->status = SEVP_MAXITER;
       return;
@@ -256,9 +276,9 @@ struct TileFin {
       st->done = 1;
       return;
     }
-    st->beta = first ? 0.0 : rz / st->rz;
-    if (st->hist && st->iter >= 1 && st->iter <= st->hist_cap)
-      st->hist[2 * (st->iter - 1) + 1] = st->beta;
+    const double next = first ? 0.0 : rz / rz_old;
+    st->beta = next;
+    if (hist && iter >= 1 && iter <= hist_cap) hist[2 * (iter - 1) + 1] = next;
     st->rz = rz;
   }
 };
@@ -577,10 +597,16 @@ int cheb_launch(const ChebLaunch<V> &L);
 // Finisher of pass A: p.q is complete; alpha = r.z / p.q.
 struct PassAFin {
   SolveState *st;
+  double rz, *hist;
+  int iter, x_pend, x_init, hist_cap;
+  __device__ void load() {
+    rz = st->rz, iter = st->iter, x_pend = st->x_pend, x_init = st->x_init;
+    hist = st->hist, hist_cap = st->hist_cap;
+  }
   __device__ void operator()(double (&s)[1]) {
     st->pq = s[0];
-    st->iter += 1;
-    if (st->x_pend) st->x_init = 1;  // this pass added the step before
+    st->iter = iter + 1;
+    st->x_init = x_pend ? 1 : x_init;  // this pass added the step before
     st->x_pend = 0;
     if (!isfinite(s[0])) {
       st->status = SEVP_NONFINITE;
@@ -589,9 +615,10 @@ struct PassAFin {
       st->status = SEVP_BREAKDOWN;
       st->done = 1;
     } else {
-      st->alpha = st->rz / s[0];
+      const double alpha = rz / s[0];
+      st->alpha = alpha;
       st->x_pend = 1;
-      if (st->hist && st->iter <= st->hist_cap) st->hist[2 * (st->iter - 1)] = st->alpha;
+      if (hist && iter + 1 <= hist_cap) hist[2 * iter] = alpha;
     }
   }
 };

@@ -70,6 +70,11 @@ struct Maps {
 // anywhere reports SEVP_TIMEOUT.
 struct TmaFin {
   SolveState *st;
+  PassAFin fin;
+  __device__ void load() {
+    fin.st = st;
+    fin.load();
+  }
   __device__ void operator()(double (&s)[2]) {
     if (s[1] != 0.0) {
       st->status = SEVP_TIMEOUT;
@@ -77,7 +82,7 @@ struct TmaFin {
       return;
     }
     double v[1] = {s[0]};
-    PassAFin{st}(v);
+    fin(v);
   }
 };
 

@@ -49,6 +49,11 @@ struct RowMaps {
 // r.z and r.r as TileFin; a failed wait anywhere reports SEVP_TIMEOUT.
 struct PassBFin {
   SolveState *st;
+  TileFin fin;
+  __device__ void load() {
+    fin.st = st;
+    fin.load();
+  }
   __device__ void operator()(double (&s)[3]) {
     if (s[2] != 0.0) {
       st->status = SEVP_TIMEOUT;
@@ -56,7 +61,7 @@ struct PassBFin {
       return;
     }
     double v[2] = {s[0], s[1]};
-    TileFin{st}(v);
+    fin(v);
   }
 };
 
