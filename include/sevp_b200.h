@@ -294,9 +294,10 @@ int sevp_set_graphs(sevp_ctx *ctx, int enable);
 int sevp_set_pass_a_kernel(sevp_ctx *ctx, int kind);
 /* Kernel of the tile passes on the block-Jacobi tiles (r -= alpha q, z =
  * M^-1 r, r.z, r.r).  SEVP_PASS_B_PAIRS (default) holds two columns per lane,
- * for FP32 and FP64 vectors, where the operator is symmetric and the
- * influence data FP64; other cases run the one-column kernels, which the
- * other two kinds always select:
+ * for FP32 and FP64 vectors, where the operator is symmetric, the influence
+ * data FP64 and the tile shape suits it (17 to 32 columns, or 8 or 16 columns
+ * with up to 8 or at least 16 rows); other cases run the one-column kernels,
+ * which the other two kinds always select:
  * SEVP_PASS_B_REGISTERS loads each task's rows and influence matrices into
  * registers when it starts (FP32 vectors, tiles of at most 6 rows; other
  * tiles march row by row); SEVP_PASS_B_STAGED has, in the FP32 PCG's tile

@@ -1255,6 +1255,22 @@ static int launch_tile_pair(sevp_ctx *ctx, const Tiling &T, V *r, const V *q, V 
   return tile_pair_launch(L);
 }
 
+// Whether the two-column pass is the faster one for a tiling.  Whole solves,
+// one-column time over two-column time on one box (FP64 / mixed), grids from
+// 150 x 80 to 2400 x 1500:
+//   32-lane segments (17 to 32 columns): 1.3 to 2.8 at every height;
+//   8 or 16 columns, up to 8 rows (in registers): 16 x 6 1.15 to 1.3, 16 x 4 and
+//     8 x 4 0.97 to 1.14; 16 rows and more (staged): 16 x 16 1.03 to 1.27;
+//   9 to 12 rows (staged, too few warps fit): 0.79 to 1.18, below 1 from
+//     1000 x 600 on: the one-column pass;
+//   narrower than their segment (12 x 6, 5 x 6): 0.84 to 1.08: the one-column
+//     pass.
+static bool pair_pass_pays(const TileGeom &tg) {
+  if (tg.hmax > kPairMaxRows) return false;
+  if (tg.wseg == 32) return true;
+  return tg.tm == tg.wseg && (tg.hmax <= kPairRegRows || tg.hmax >= 16);
+}
+
 // Dispatch: symmetric-coefficient variant when the operator is symmetric;
 // FP32 influence matrices only for FP32 vectors when the solve asks for them.
 template <typename V, bool UPDATE, bool DOTS>
@@ -1272,7 +1288,7 @@ static int launch_tile(sevp_ctx *ctx, const Tiling &T, V *r, const V *q, V *z, i
       return launch_tile_k<V, MixMat, UPDATE, DOTS, false>(ctx, T, mm, r, q, z, ticket_slot);
     }
   }
-  if (ctx->sym && ctx->pass_b_kernel == SEVP_PASS_B_PAIRS && T.tg.hmax <= kPairMaxRows)
+  if (ctx->sym && ctx->pass_b_kernel == SEVP_PASS_B_PAIRS && pair_pass_pays(T.tg))
     return launch_tile_pair<V, UPDATE, DOTS>(ctx, T, r, q, z, ticket_slot);
   if (ctx->sym)
     return launch_tile_k<V, double, UPDATE, DOTS, true>(ctx, T, T.d_mats, r, q, z, ticket_slot);
