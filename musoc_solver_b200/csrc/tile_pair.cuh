@@ -611,15 +611,19 @@ int tile_pair_launch_k(const PairLaunch<V> &L) {
   const TileGeom &tg = L.tg;
   const size_t per_warp = pair_smem_per_warp<V, W, HM>(tg.nbmax);
   // CTA size (in warps) with the most resident warps, and its resident CTAs,
-  // for the last shared-memory size (contexts in several threads may differ
-  // in sub-block counts)
+  // per sub-block count (the shared memory depends on nothing else)
+  struct Fit {
+    int warps = 0, slots = 0;
+  };
   static std::mutex mu;
-  static size_t set_smem = 0;
-  static int best_warps = 1, slots = 1, sms = 1;
-  int use_warps, use_slots, use_sms;
+  static Fit fits[kPairMaxRows + 1];
+  static int sms = 0;
+  Fit fit;
+  int use_sms;
   {
     std::lock_guard<std::mutex> lock(mu);
-    if (set_smem != per_warp) {
+    Fit &f = fits[tg.nbmax];
+    if (!f.warps) {
       int dev = 0, optin = 0, best = 0;
       SEVP_CUDA_TRY(cudaGetDevice(&dev));
       SEVP_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
@@ -627,25 +631,26 @@ int tile_pair_launch_k(const PairLaunch<V> &L) {
       const size_t room = (size_t)optin - 1024;  // static shared memory of the sums
       SEVP_CUDA_TRY(
           cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)room));
+      Fit found;
       for (int w = kPairWarps; w >= 1; --w) {
         int per_sm = 0;
         if (per_warp * w > room) continue;
         SEVP_CUDA_TRY(
             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, w * 32, per_warp * w));
-        if (per_sm * w > best) best = per_sm * w, best_warps = w, slots = per_sm * sms;
+        if (per_sm * w > best) best = per_sm * w, found.warps = w, found.slots = per_sm * sms;
       }
       if (!best) {
         sevp_internal_set_message("tile pass: a warp's rows do not fit the shared memory");
         return SEVP_BAD_ARG;
       }
-      set_smem = per_warp;
+      f = found;
     }
-    use_warps = best_warps, use_slots = slots, use_sms = sms;
+    fit = f, use_sms = sms;
   }
   const long long ntasks = (long long)tg.ty * pair_cols(tg);
   // few tasks: fewer warps per CTA, so that they spread over the SMs
-  const int warps = (int)std::min<long long>(use_warps, std::max<long long>(1, ntasks / use_sms));
-  const long long want = std::min<long long>((ntasks + warps - 1) / warps, use_slots);
+  const int warps = (int)std::min<long long>(fit.warps, std::max<long long>(1, ntasks / use_sms));
+  const long long want = std::min<long long>((ntasks + warps - 1) / warps, fit.slots);
   const unsigned blocks =
       (unsigned)std::max<long long>(1, std::min<long long>(want, (long long)(L.partials_n / 2)));
   // vector copies: every lane's first column is even, its pair in one row, and
