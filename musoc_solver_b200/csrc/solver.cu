@@ -1256,7 +1256,7 @@ static int launch_tile_pair(sevp_ctx *ctx, const Tiling &T, V *r, const V *q, V 
 }
 
 // Whether the two-column pass is the faster one for a tiling.  Whole solves,
-// one-column time over two-column time on one box (FP64 / mixed), grids from
+// one-column time over two-column time on one B200 (FP64 / mixed), grids from
 // 150 x 80 to 2400 x 1500:
 //   32-lane segments (17 to 32 columns): 1.3 to 2.8 at every height;
 //   8 or 16 columns, up to 8 rows (in registers): 16 x 6 1.15 to 1.3, 16 x 4 and

@@ -31,7 +31,7 @@
 // fill the memory (one SM's warps move 6.2 TB/s / 148 between their first and
 // last task; the slowest SM ends 18 % after the median one, and handing out
 // the last tasks from a counter cost more in their sums than it gained).
-// Measured at 3600 x 2400, 16 x 6 tiles, one box: FP32 138 -> 101 us (481 MB,
+// Measured at 3600 x 2400, 16 x 6 tiles, one B200: FP32 138 -> 101 us (481 MB,
 // 4.8 TB/s), FP64 179 -> 127 us; 1440 x 720 FP64 35.6 -> 27.8 us.
 #pragma once
 #include "solver_core.cuh"
