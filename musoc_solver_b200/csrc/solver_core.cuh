@@ -237,6 +237,18 @@ __device__ __forceinline__ double march_rcp(double a) {
   return fma(r, e, r);
 }
 
+// q / a of a marching row with rcp = march_rcp(a) formed ahead.  FP32 vectors
+// take the product: z is rounded to FP32.  FP64 vectors add one Newton step
+// on the quotient, t + rcp (q - a t), whose remainder is exact in a fused
+// multiply-add (P. Markstein, IBM J. Res. Dev. 34(1), 1990): the rounded
+// quotient, as a division gives, for two more operations on the row's chain.
+template <typename V>
+__device__ __forceinline__ double march_quot(double q, double a, double rcp) {
+  const double t = q * rcp;
+  if (sizeof(V) == 4) return t;
+  return fma(fma(-a, t, q), rcp, t);
+}
+
 // Finishes a PCG iteration after pass B: r.z and r.r are complete.
 struct TileFin {
   SolveState *st;

@@ -27,12 +27,18 @@
 //     influence matrix gives (z_{k+1} from r_k, z_{k-1}, z_k) instead of
 //     marching a homogeneous correction and adding it to stored rows: the
 //     same error (that of the guess row times the growth), no stored rows.
+//     FP64 quotients are rounded as a division's (march_quot).  Error of z in
+//     FP64 against refined dense solves of up to 6000 tiles, as a part of the
+//     one-column pass's (geometric mean over the tiles; rms): 16 x 6 tiles of
+//     1440 x 720 0.99; 0.98, 16 x 16 of 1203 x 601 0.99; 0.94, 32 x 8, 8 x 8
+//     and 16 x 4 of 600 x 300 1.01; 1.05, 1.02; 1.04 and 1.00; 0.96.
 // Two CTAs of four warps per SM: three spill, and the loads in flight already
 // fill the memory (one SM's warps move 6.2 TB/s / 148 between their first and
 // last task; the slowest SM ends 18 % after the median one, and handing out
 // the last tasks from a counter cost more in their sums than it gained).
 // Measured at 3600 x 2400, 16 x 6 tiles, one B200: FP32 138 -> 101 us (481 MB,
-// 4.8 TB/s), FP64 179 -> 127 us; 1440 x 720 FP64 35.6 -> 27.8 us.
+// 4.8 TB/s), FP64 179 -> 128 us; 1440 x 720 FP64 35.6 -> 28.3 us (of which
+// the rounded quotients 1 us and 0.5 us).
 #pragma once
 #include "solver_core.cuh"
 
@@ -373,8 +379,12 @@ __global__ void __launch_bounds__(kPairWarps * 32, 2)
             acc_rr += a1 * a1;
           }
         }
-        // row k's equation residual with the rows below (zb, zc); the terms
-        // that wait on the neighbour shuffles come last
+        // row k's equation residual with the rows below (zb, zc): two of the
+        // three neighbours before the centre, which has the other sign, so
+        // that the partial sums stay as small as they do from west to east
+        // (8 x 8 tiles of 600 x 300, FP64: error of z 1.06 times as large
+        // with the centre ahead of both columns); the term that waits on the
+        // neighbour shuffles last
         auto row = [&](int k, bool first, bool second, double zb0, double zb1, double zc0,
                        double zc1, double &q0, double &q1) {
           double p0 = (double)r0[k], p1 = (double)r1[k];
@@ -386,10 +396,10 @@ __global__ void __launch_bounds__(kPairWarps * 32, 2)
               p1 -= (double)cn1[k > 0 ? k - 1 : 0] * zb1;
             }
             const double e0 = (double)ce0[k];
-            p0 -= (double)cc0[k] * zc0;
-            p1 -= (double)cc1[k] * zc1;
             p0 -= e0 * zc1;
             p1 -= e0 * zc0;
+            p0 -= (double)cc0[k] * zc0;
+            p1 -= (double)cc1[k] * zc1;
             p0 -= (double)cw0[k] * zw;
             p1 -= (double)ce1[k] * ze;
           }
@@ -401,8 +411,8 @@ __global__ void __launch_bounds__(kPairWarps * 32, 2)
           row(k, k == 0, k == 1, zb0, zb1, zc0, zc1, q0, q1);
           if (k < HM - 1) {
             zb0 = zc0, zb1 = zc1;
-            zc0 = q0 * march_rcp((double)cn0[k]);
-            zc1 = q1 * march_rcp((double)cn1[k]);
+            zc0 = march_quot<V>(q0, (double)cn0[k], march_rcp((double)cn0[k]));
+            zc1 = march_quot<V>(q1, (double)cn1[k], march_rcp((double)cn1[k]));
           }
         }
         __syncwarp();
@@ -419,8 +429,8 @@ __global__ void __launch_bounds__(kPairWarps * 32, 2)
         for (int k = 0; k < HM - 1; ++k) {
           row(k, false, k == 0, zb0, zb1, zc0, zc1, q0, q1);
           zb0 = zc0, zb1 = zc1;
-          zc0 = q0 * march_rcp((double)cn0[k]);
-          zc1 = q1 * march_rcp((double)cn1[k]);
+          zc0 = march_quot<V>(q0, (double)cn0[k], march_rcp((double)cn0[k]));
+          zc1 = march_quot<V>(q1, (double)cn1[k], march_rcp((double)cn1[k]));
           emit(k + 1, zc0, zc1);
         }
         ran = true;
@@ -456,9 +466,9 @@ __global__ void __launch_bounds__(kPairWarps * 32, 2)
       }
       // Row k's coefficients and right-hand side, converted, and its
       // reciprocals of AT: taken one row ahead of the march, so that only the
-      // shuffles, one multiply-add and a multiply are on its chain.
+      // shuffles, one multiply-add and the quotient are on its chain.
       struct RowC {
-        double s0, s1, f0, f1, e0, e1, w0, i0, i1, p0, p1;
+        double s0, s1, f0, f1, e0, e1, w0, n0, n1, i0, i1, p0, p1;
       };
       auto take = [&](int k) {
         RowC c;
@@ -472,8 +482,8 @@ __global__ void __launch_bounds__(kPairWarps * 32, 2)
         c.s0 = (double)s0, c.s1 = (double)s1, c.f0 = (double)f0, c.f1 = (double)f1;
         c.e0 = (double)e0, c.e1 = (double)e1, c.w0 = (double)w0;
         c.p0 = (double)wr[k * kR], c.p1 = (double)wr[k * kR + 1];
-        c.i0 = march_rcp(c0 ? (double)n0 : 1.0);
-        c.i1 = march_rcp(c1 ? (double)n1 : 1.0);
+        c.n0 = c0 ? (double)n0 : 1.0, c.n1 = c1 ? (double)n1 : 1.0;
+        c.i0 = march_rcp(c.n0), c.i1 = march_rcp(c.n1);
         return c;
       };
       auto row = [&](const RowC &c, double zb0, double zb1, double zc0, double zc1, double &q0,
@@ -481,10 +491,10 @@ __global__ void __launch_bounds__(kPairWarps * 32, 2)
         const double zw = __shfl_up_sync(0xffffffffu, zc1, 1, LPT);
         const double ze = __shfl_down_sync(0xffffffffu, zc0, 1, LPT);
         double p0 = c.p0 - c.s0 * zb0, p1 = c.p1 - c.s1 * zb1;
-        p0 -= c.f0 * zc0;
-        p1 -= c.f1 * zc1;
         p0 -= c.e0 * zc1;
         p1 -= c.e0 * zc0;
+        p0 -= c.f0 * zc0;
+        p1 -= c.f1 * zc1;
         p0 -= c.w0 * zw;
         p1 -= c.e1 * ze;
         q0 = p0, q1 = p1;
@@ -504,7 +514,7 @@ __global__ void __launch_bounds__(kPairWarps * 32, 2)
           const bool last = k == ke, fix = last && t < nb - 1;
           if (last) rho[t * 32] = make_double2(q0, q1);
           zb0 = zc0, zb1 = zc1;
-          if (!last) zc0 = q0 * c.i0, zc1 = q1 * c.i1;
+          if (!last) zc0 = march_quot<V>(q0, c.n0, c.i0), zc1 = march_quot<V>(q1, c.n1, c.i1);
           c = cn;
           if (__any_sync(0xffffffffu, fix)) {
             __syncwarp();
@@ -586,7 +596,7 @@ __global__ void __launch_bounds__(kPairWarps * 32, 2)
           row(c, zb0, zb1, zc0, zc1, q0, q1);
           if (in && k < ke) {
             zb0 = zc0, zb1 = zc1;
-            zc0 = q0 * c.i0, zc1 = q1 * c.i1;
+            zc0 = march_quot<V>(q0, c.n0, c.i0), zc1 = march_quot<V>(q1, c.n1, c.i1);
           }
           c = cn;
         }
