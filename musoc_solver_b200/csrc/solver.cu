@@ -345,8 +345,10 @@ __device__ __forceinline__ void load_row(RowIn<V> &in, const Coeffs &c, const V 
   in.cn = __ldg(c.at + idx);
 }
 
-// UPDATE: fused r -= alpha q before preconditioning (pass B).  DOTS without
-//         UPDATE starts a run, and is skipped by one that resumes.
+// st:     the run's state; a launch of a finished run returns at once.  Null
+//         outside a solve (neither UPDATE nor DOTS).
+// UPDATE: fused r -= alpha q before preconditioning (pass B).  Without
+//         UPDATE the launch starts a run, and is skipped by one that resumes.
 // DOTS:   accumulate r.z and r.r and finish the iteration on the device.
 // SYM:    symmetric operator: AL and AB are taken from the west lane's AR and
 //         the previous row's AT (inside a tile the couplings that cross the
@@ -357,7 +359,7 @@ template <typename V, typename MT, bool UPDATE, bool DOTS, bool SYM>
 __global__ void __launch_bounds__(kTileWarps * 32, SEVP_TILE_MINB)
     k_tile_apply(TileGeom tg, Coeffs c, const MT *__restrict__ mats, V *r, const V *q, V *z,
                  SolveState *st, double *partials, unsigned *ticket) {
-  if ((DOTS || UPDATE) && (st->done || (!UPDATE && st->resumed))) return;
+  if (st && (st->done || (!UPDATE && st->resumed))) return;
   constexpr bool kChain = sizeof(V) == 4;
   extern __shared__ __align__(16) unsigned char tsm[];
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
@@ -548,7 +550,7 @@ template <typename V, typename MT, bool UPDATE, bool DOTS, bool SYM, int HM>
 __global__ void __launch_bounds__(kTileWarps * 32, 2)
     k_tile_short(TileGeom tg, Coeffs c, const MT *__restrict__ mats, V *r, const V *q, V *z,
                  SolveState *st, double *partials, unsigned *ticket) {
-  if ((DOTS || UPDATE) && (st->done || (!UPDATE && st->resumed))) return;
+  if (st && (st->done || (!UPDATE && st->resumed))) return;
   constexpr bool kChain = sizeof(V) == 4;
   __shared__ double dv_all[kTileWarps * 32];
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
@@ -1207,7 +1209,7 @@ static int resident_ctas(K kern, size_t smem, size_t &set_smem, int &slots) {
 
 template <typename V, typename MT, bool UPDATE, bool DOTS, bool SYM>
 static int launch_tile_k(sevp_ctx *ctx, const Tiling &T, const MT *mats, V *r, const V *q, V *z,
-                         int ticket_slot) {
+                         SolveState *st, int ticket_slot) {
   const size_t warps = tile_warps(T.tg);
   const bool short_tiles = sizeof(V) == 4 && T.tg.hmax <= kShortTileRows;
   const size_t smem = short_tiles ? 0 : tile_smem_per_warp(T.tg.hmax) * kTileWarps;
@@ -1236,7 +1238,7 @@ static int launch_tile_k(sevp_ctx *ctx, const Tiling &T, const MT *mats, V *r, c
     ctx->pass_b_used = SEVP_PASS_B_REGISTERS;
   }
   ProfScope ps(ctx, UPDATE ? 0 : 2);
-  kern<<<blocks, kTileWarps * 32, smem, ctx->stream>>>(T.tg, T.c, mats, r, q, z, ctx->st,
+  kern<<<blocks, kTileWarps * 32, smem, ctx->stream>>>(T.tg, T.c, mats, r, q, z, st,
                                                       ctx->partials, ctx->tickets + ticket_slot);
   ctx->launches++;
   SEVP_CUDA_TRY(cudaGetLastError());
@@ -1246,10 +1248,10 @@ static int launch_tile_k(sevp_ctx *ctx, const Tiling &T, const MT *mats, V *r, c
 // Two-column tile pass (tile_pair.cuh).
 template <typename V, bool UPDATE, bool DOTS>
 static int launch_tile_pair(sevp_ctx *ctx, const Tiling &T, V *r, const V *q, V *z,
-                            int ticket_slot) {
+                            SolveState *st, int ticket_slot) {
   if (sizeof(V) == 4 && UPDATE && DOTS) ctx->pass_b_used = SEVP_PASS_B_PAIRS;
   ProfScope ps(ctx, UPDATE ? 0 : 2);
-  const PairLaunch<V> L{T.tg, T.c, T.d_mats, r, q, z, ctx->st, ctx->partials, ctx->partials_n,
+  const PairLaunch<V> L{T.tg, T.c, T.d_mats, r, q, z, st, ctx->partials, ctx->partials_n,
                         ctx->tickets + ticket_slot, ctx->stream, UPDATE, DOTS};
   ctx->launches++;
   return tile_pair_launch(L);
@@ -1273,26 +1275,30 @@ static bool pair_pass_pays(const TileGeom &tg) {
 
 // Dispatch: symmetric-coefficient variant when the operator is symmetric;
 // FP32 influence matrices only for FP32 vectors when the solve asks for them.
+// st: the run's state inside a solve, else null.
 template <typename V, bool UPDATE, bool DOTS>
-static int launch_tile(sevp_ctx *ctx, const Tiling &T, V *r, const V *q, V *z, int ticket_slot) {
+static int launch_tile(sevp_ctx *ctx, const Tiling &T, V *r, const V *q, V *z, SolveState *st,
+                       int ticket_slot) {
   if constexpr (sizeof(V) == 4) {
     if (ctx->infl32_active && T.d_mats32) {
       if (ctx->sym)
-        return launch_tile_k<V, float, UPDATE, DOTS, true>(ctx, T, T.d_mats32, r, q, z, ticket_slot);
-      return launch_tile_k<V, float, UPDATE, DOTS, false>(ctx, T, T.d_mats32, r, q, z, ticket_slot);
+        return launch_tile_k<V, float, UPDATE, DOTS, true>(ctx, T, T.d_mats32, r, q, z, st,
+                                                             ticket_slot);
+      return launch_tile_k<V, float, UPDATE, DOTS, false>(ctx, T, T.d_mats32, r, q, z, st,
+                                                           ticket_slot);
     }
     if (T.d_matsmix && T.f32_groups > 0) {  // without FP32 groups: the FP64 data itself
       const MixMat *mm = reinterpret_cast<const MixMat *>(T.d_matsmix);
       if (ctx->sym)
-        return launch_tile_k<V, MixMat, UPDATE, DOTS, true>(ctx, T, mm, r, q, z, ticket_slot);
-      return launch_tile_k<V, MixMat, UPDATE, DOTS, false>(ctx, T, mm, r, q, z, ticket_slot);
+        return launch_tile_k<V, MixMat, UPDATE, DOTS, true>(ctx, T, mm, r, q, z, st, ticket_slot);
+      return launch_tile_k<V, MixMat, UPDATE, DOTS, false>(ctx, T, mm, r, q, z, st, ticket_slot);
     }
   }
   if (ctx->sym && ctx->pass_b_kernel == SEVP_PASS_B_PAIRS && pair_pass_pays(T.tg))
-    return launch_tile_pair<V, UPDATE, DOTS>(ctx, T, r, q, z, ticket_slot);
+    return launch_tile_pair<V, UPDATE, DOTS>(ctx, T, r, q, z, st, ticket_slot);
   if (ctx->sym)
-    return launch_tile_k<V, double, UPDATE, DOTS, true>(ctx, T, T.d_mats, r, q, z, ticket_slot);
-  return launch_tile_k<V, double, UPDATE, DOTS, false>(ctx, T, T.d_mats, r, q, z, ticket_slot);
+    return launch_tile_k<V, double, UPDATE, DOTS, true>(ctx, T, T.d_mats, r, q, z, st, ticket_slot);
+  return launch_tile_k<V, double, UPDATE, DOTS, false>(ctx, T, T.d_mats, r, q, z, st, ticket_slot);
 }
 
 // Tile rows the Schwarz stage kernel holds in registers.
@@ -1361,12 +1367,12 @@ static void schwarz_bufs(sevp_ctx *ctx, V *&s1, V *&s2) {
 // A (z1 + z2)), the residuals formed from the tile-boundary couplings.
 template <typename V, bool UPDATE, bool DOTS>
 static int precondition_pass(sevp_ctx *ctx, V *r, const V *q, V *z) {
-  if (!schwarz_on(ctx)) return launch_tile<V, UPDATE, DOTS>(ctx, ctx->ta, r, q, z, 4);
+  SolveState *st = UPDATE || DOTS ? ctx->st : nullptr;
+  if (!schwarz_on(ctx)) return launch_tile<V, UPDATE, DOTS>(ctx, ctx->ta, r, q, z, st, 4);
   V *s1, *s2;
   schwarz_bufs(ctx, s1, s2);
-  int s = launch_tile<V, UPDATE, false>(ctx, ctx->ta, r, q, s1, 4);
+  int s = launch_tile<V, UPDATE, false>(ctx, ctx->ta, r, q, s1, st, 4);
   if (s) return s;
-  SolveState *st = DOTS ? ctx->st : nullptr;
   s = launch_couple<V, 0>(ctx, ctx->tb, ctx->ta.tg.xs, s1, nullptr, nullptr, s2, st, 4);
   if (s) return s;
   if (DOTS) return launch_couple<V, 2>(ctx, ctx->ta, ctx->tb.tg.xs, s2, s1, r, z, ctx->st, 4);
@@ -2927,7 +2933,7 @@ extern "C" int sevp_nn_features(sevp_ctx *ctx, const double *eta1, const double 
   if (s) return s;
   // the feature is the block-Jacobi preconditioner's response (what the
   // network was trained on), whichever preconditioner the solves use
-  s = launch_tile<double, false, false>(ctx, ctx->ta, ctx->r64, nullptr, m, 1);
+  s = launch_tile<double, false, false>(ctx, ctx->ta, ctx->r64, nullptr, m, nullptr, 1);
   if (s) return s;
   SEVP_CUDA_TRY(cudaMemsetAsync(ctx->nn_avg, 0, 3 * nn * sizeof(float), ctx->stream));
   const dim3 pgrid((unsigned)ceil_div(ctx->nx / coarse * coarse, kPackThreads),

@@ -694,7 +694,7 @@ struct PairLaunch {
   V *r;
   const V *q;
   V *z;
-  SolveState *st;
+  SolveState *st;  // null outside a solve (neither update nor dots)
   double *partials;
   size_t partials_n;  // doubles in partials (two per CTA are used)
   unsigned *ticket;

@@ -290,7 +290,7 @@ __global__ void __launch_bounds__(kPairWarps * 32, 2)
   pdl_wait();
   // a finished run's launches, and the start pass of a run that resumes, end
   // here (tested once the first copies are under way)
-  const int done = (DOTS || UPDATE) ? st->done || (!UPDATE && st->resumed) : 0;
+  const int done = st ? st->done || (!UPDATE && st->resumed) : 0;
   const V alpha = UPDATE ? (V)st->alpha : V(0);
   if (pos < ntasks) {
     fetch_vectors(nxt);
