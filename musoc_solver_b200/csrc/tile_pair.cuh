@@ -620,10 +620,11 @@ int tile_pair_launch_k(const PairLaunch<V> &L) {
   auto kern = k_tile_pair<V, W, HM, UPDATE, DOTS>;
   const TileGeom &tg = L.tg;
   const size_t per_warp = pair_smem_per_warp<V, W, HM>(tg.nbmax);
-  // CTA size (in warps) with the most resident warps, and its resident CTAs,
-  // per sub-block count (the shared memory depends on nothing else)
+  // resident CTAs by CTA size (in warps), per sub-block count (the shared
+  // memory depends on nothing else)
   struct Fit {
-    int warps = 0, slots = 0;
+    int slots[kPairWarps + 1] = {};
+    int best = 0;  // the CTA size with the most resident warps
   };
   static std::mutex mu;
   static Fit fits[kPairMaxRows + 1];
@@ -633,8 +634,8 @@ int tile_pair_launch_k(const PairLaunch<V> &L) {
   {
     std::lock_guard<std::mutex> lock(mu);
     Fit &f = fits[tg.nbmax];
-    if (!f.warps) {
-      int dev = 0, optin = 0, best = 0;
+    if (!f.best) {
+      int dev = 0, optin = 0;
       SEVP_CUDA_TRY(cudaGetDevice(&dev));
       SEVP_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
       SEVP_CUDA_TRY(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
@@ -647,9 +648,10 @@ int tile_pair_launch_k(const PairLaunch<V> &L) {
         if (per_warp * w > room) continue;
         SEVP_CUDA_TRY(
             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, w * 32, per_warp * w));
-        if (per_sm * w > best) best = per_sm * w, found.warps = w, found.slots = per_sm * sms;
+        found.slots[w] = per_sm * sms;
+        if (found.slots[w] * w > found.slots[found.best] * found.best) found.best = w;
       }
-      if (!best) {
+      if (!found.best) {
         sevp_internal_set_message("tile pass: a warp's rows do not fit the shared memory");
         return SEVP_BAD_ARG;
       }
@@ -658,9 +660,13 @@ int tile_pair_launch_k(const PairLaunch<V> &L) {
     fit = f, use_sms = sms;
   }
   const long long ntasks = (long long)tg.ty * pair_cols(tg);
-  // few tasks: fewer warps per CTA, so that they spread over the SMs
-  const int warps = (int)std::min<long long>(fit.warps, std::max<long long>(1, ntasks / use_sms));
-  const long long want = std::min<long long>((ntasks + warps - 1) / warps, fit.slots);
+  // few tasks: fewer warps per CTA, so that they spread over the SMs, where
+  // all tasks are then resident at once (a second round doubles the pass: 16 x
+  // 16 tiles at 592 x 344, FP64, 220 tasks on 148 one-warp CTAs: 45 us, on 220:
+  // 27 us)
+  int warps = (int)std::min<long long>(fit.best, std::max<long long>(1, ntasks / use_sms));
+  if ((long long)fit.slots[warps] * warps < ntasks) warps = fit.best;
+  const long long want = std::min<long long>((ntasks + warps - 1) / warps, fit.slots[warps]);
   const unsigned blocks =
       (unsigned)std::max<long long>(1, std::min<long long>(want, (long long)(L.partials_n / 2)));
   // vector copies: every lane's first column is even, its pair in one row, and
@@ -675,8 +681,8 @@ int tile_pair_launch_k(const PairLaunch<V> &L) {
   // a solve's kernels only: the planes are read before the kernel ahead has
   // ended, and outside a solve that kernel may be the caller's, writing them
   SEVP_CUDA_TRY(launch_overlapped(kern, blocks, warps * 32, per_warp * warps, L.stream,
-                                  UPDATE || DOTS, tg, L.c.ac, L.c.ar, L.c.at, L.mats, L.r, L.q, L.z, L.st, L.partials,
-                                  L.ticket, quad ? 2 : (vec ? 1 : 0)));
+                                  UPDATE || DOTS, tg, L.c.ac, L.c.ar, L.c.at, L.mats, L.r, L.q,
+                                  L.z, L.st, L.partials, L.ticket, quad ? 2 : (vec ? 1 : 0)));
   return SEVP_OK;
 }
 
