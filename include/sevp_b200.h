@@ -295,8 +295,9 @@ int sevp_set_pass_a_kernel(sevp_ctx *ctx, int kind);
 /* Kernel of the tile passes on the block-Jacobi tiles (r -= alpha q, z =
  * M^-1 r, r.z, r.r).  SEVP_PASS_B_PAIRS (default) holds two columns per lane,
  * for FP32 and FP64 vectors, where the operator is symmetric, the influence
- * data FP64 and the tile shape suits it (17 to 32 columns, or 8 or 16 columns
- * with up to 8 or at least 16 rows); other cases run the one-column kernels,
+ * data FP64 and it is the faster one for the tiling (17 to 32 columns, or 8 or
+ * 16 columns with 3 to 8 or at least 16 rows, unless only its tasks need a
+ * second round of resident warps); other cases run the one-column kernels,
  * which the other two kinds always select:
  * SEVP_PASS_B_REGISTERS loads each task's rows and influence matrices into
  * registers when it starts (FP32 vectors, tiles of at most 6 rows; other
@@ -325,6 +326,11 @@ int sevp_set_resume_check(sevp_ctx *ctx, double max_rel_dev);
  * SEVP_PASS_B_STAGED or SEVP_PASS_B_PAIRS, -1 before the first.  Test hook; not part of the
  * reference interface. */
 int sevp_pass_b_kernel_used(const sevp_ctx *ctx);
+/* The same for the context's last tile pass of any kind and precision
+ * (sevp_precondition, a run's start and its iterations; one-column passes
+ * count as SEVP_PASS_B_REGISTERS).  Test hook; not part of the reference
+ * interface. */
+int sevp_tile_kernel_used(const sevp_ctx *ctx);
 /* One stencil pass on caller device buffers with the context's operator and
  * pass A kernel: p = z + beta p_old (z alone when beta == 0), q = A p, and
  * p.q through pq_out.  Test hook; not part of the reference interface. */

@@ -975,6 +975,8 @@ struct Tiling {
   std::vector<int> grp_nb;   // per warp group (ty * txg)
   std::vector<int> tile_nb;  // effective sub-blocks per tile (ty * tx)
   bool built = false;
+  // whether the two-column pass runs (FP32, FP64 vectors; -1: not asked yet)
+  mutable signed char pair_choice[2] = {-1, -1};
   void release() {
     for (void *p : {(void *)d_grp_nb, (void *)d_moff, (void *)d_mats, (void *)d_mats32,
                     (void *)d_al, (void *)d_ar, (void *)d_matsmix, (void *)d_grp_f32,
@@ -988,6 +990,7 @@ struct Tiling {
     mix_bytes_per_pass = 0;
     mats_elems = 0;
     built = false;
+    pair_choice[0] = pair_choice[1] = -1;
   }
 };
 
@@ -1076,6 +1079,7 @@ struct sevp_ctx {
   int pass_a_kernel = SEVP_PASS_A_TILES;
   int pass_b_kernel = SEVP_PASS_B_PAIRS;
   int pass_b_used = -1;  // kernel of the last FP32 pass B launch
+  int tile_used = -1;    // kernel of the last tile pass of any kind
   cudaStream_t cap_stream = nullptr;
   cudaGraphExec_t inner_graph = nullptr;
   int inner_graph_ce = 0;
@@ -1207,21 +1211,40 @@ static int resident_ctas(K kern, size_t smem, size_t &set_smem, int &slots) {
   return SEVP_OK;
 }
 
+// Whether the one-column pass of a tiling is the register kernel.
+template <typename V>
+static bool tile_is_short(const TileGeom &tg) {
+  return sizeof(V) == 4 && tg.hmax <= kShortTileRows;
+}
+
+// Resident CTAs of the one-column pass.
 template <typename V, typename MT, bool UPDATE, bool DOTS, bool SYM>
-static int launch_tile_k(sevp_ctx *ctx, const Tiling &T, const MT *mats, V *r, const V *q, V *z,
-                         SolveState *st, int ticket_slot) {
-  const size_t warps = tile_warps(T.tg);
-  const bool short_tiles = sizeof(V) == 4 && T.tg.hmax <= kShortTileRows;
-  const size_t smem = short_tiles ? 0 : tile_smem_per_warp(T.tg.hmax) * kTileWarps;
+static int one_column_slots(const TileGeom &tg, int &slots) {
+  const bool short_tiles = tile_is_short<V>(tg);
+  const size_t smem = short_tiles ? 0 : tile_smem_per_warp(tg.hmax) * kTileWarps;
   auto kern = short_tiles ? k_tile_short<V, MT, UPDATE, DOTS, SYM, kShortTileRows>
                           : k_tile_apply<V, MT, UPDATE, DOTS, SYM>;
   // per instantiation and kernel choice
   static size_t set_smem[2] = {0, 0};
-  static int slots[2] = {0, 0};
-  int s = resident_ctas(kern, smem, set_smem[short_tiles], slots[short_tiles]);
+  static int have[2] = {0, 0};
+  const int s = resident_ctas(kern, smem, set_smem[short_tiles], have[short_tiles]);
+  slots = have[short_tiles];
+  return s;
+}
+
+template <typename V, typename MT, bool UPDATE, bool DOTS, bool SYM>
+static int launch_tile_k(sevp_ctx *ctx, const Tiling &T, const MT *mats, V *r, const V *q, V *z,
+                         SolveState *st, int ticket_slot) {
+  const size_t warps = tile_warps(T.tg);
+  const bool short_tiles = tile_is_short<V>(T.tg);
+  const size_t smem = short_tiles ? 0 : tile_smem_per_warp(T.tg.hmax) * kTileWarps;
+  auto kern = short_tiles ? k_tile_short<V, MT, UPDATE, DOTS, SYM, kShortTileRows>
+                          : k_tile_apply<V, MT, UPDATE, DOTS, SYM>;
+  int slots = 0;
+  int s = one_column_slots<V, MT, UPDATE, DOTS, SYM>(T.tg, slots);
   if (s) return s;
-  const unsigned blocks = (unsigned)std::min<size_t>((warps + kTileWarps - 1) / kTileWarps,
-                                                     (size_t)slots[short_tiles]);
+  const unsigned blocks =
+      (unsigned)std::min<size_t>((warps + kTileWarps - 1) / kTileWarps, (size_t)slots);
   if constexpr (sizeof(V) == 4 && std::is_same<MT, double>::value && UPDATE && DOTS && SYM) {
     // PCG pass B with tensor-copied task stages, on the same grid
     if (short_tiles && ctx->pass_b_kernel == SEVP_PASS_B_STAGED) {
@@ -1231,12 +1254,13 @@ static int launch_tile_k(sevp_ctx *ctx, const Tiling &T, const MT *mats, V *r, c
         ProfScope ps(ctx, 0);
         const int s2 = pass_b_tma_launch(L);
         ctx->launches++;
-        ctx->pass_b_used = SEVP_PASS_B_STAGED;
+        ctx->pass_b_used = ctx->tile_used = SEVP_PASS_B_STAGED;
         return s2;
       }
     }
     ctx->pass_b_used = SEVP_PASS_B_REGISTERS;
   }
+  ctx->tile_used = SEVP_PASS_B_REGISTERS;
   ProfScope ps(ctx, UPDATE ? 0 : 2);
   kern<<<blocks, kTileWarps * 32, smem, ctx->stream>>>(T.tg, T.c, mats, r, q, z, st,
                                                       ctx->partials, ctx->tickets + ticket_slot);
@@ -1250,6 +1274,7 @@ template <typename V, bool UPDATE, bool DOTS>
 static int launch_tile_pair(sevp_ctx *ctx, const Tiling &T, V *r, const V *q, V *z,
                             SolveState *st, int ticket_slot) {
   if (sizeof(V) == 4 && UPDATE && DOTS) ctx->pass_b_used = SEVP_PASS_B_PAIRS;
+  ctx->tile_used = SEVP_PASS_B_PAIRS;
   ProfScope ps(ctx, UPDATE ? 0 : 2);
   const PairLaunch<V> L{T.tg, T.c, T.d_mats, r, q, z, st, ctx->partials, ctx->partials_n,
                         ctx->tickets + ticket_slot, ctx->stream, UPDATE, DOTS};
@@ -1257,20 +1282,69 @@ static int launch_tile_pair(sevp_ctx *ctx, const Tiling &T, V *r, const V *q, V 
   return tile_pair_launch(L);
 }
 
-// Whether the two-column pass is the faster one for a tiling.  Whole solves,
-// one-column time over two-column time on one B200 (FP64 / mixed), grids from
-// 150 x 80 to 2400 x 1500:
-//   32-lane segments (17 to 32 columns): 1.3 to 2.8 at every height;
-//   8 or 16 columns, up to 8 rows (in registers): 16 x 6 1.15 to 1.3, 16 x 4 and
-//     8 x 4 0.97 to 1.14; 16 rows and more (staged): 16 x 16 1.03 to 1.27;
-//   9 to 12 rows (staged, too few warps fit): 0.79 to 1.18, below 1 from
-//     1000 x 600 on: the one-column pass;
-//   narrower than their segment (12 x 6, 5 x 6): 0.84 to 1.08: the one-column
-//     pass.
-static bool pair_pass_pays(const TileGeom &tg) {
-  if (tg.hmax > kPairMaxRows) return false;
-  if (tg.wseg == 32) return true;
-  return tg.tm == tg.wseg && (tg.hmax <= kPairRegRows || tg.hmax >= 16);
+// Whether the two-column pass is the faster one for a tiling.  Numbers: whole
+// solves, one-column time over two-column time on one B200 (FP64 and mixed),
+// sixteen grids from 90 x 45 to 3600 x 2400, 103 tile shapes.
+//
+// Its warps hold two tasks' columns, so it takes half as many, but they need
+// more registers and shared memory: it holds 1/2 to 1/6 of the one-column
+// pass's warps.  While all its tasks are resident it is the faster one; where
+// they take a second round and the one-column pass's still fit one, the
+// second round costs more than the two columns gain on small tiles.
+//   32-lane segments (17 to 32 columns): 1.0 to 2.5 with all tasks resident
+//     and with several rounds on both sides, in between 0.86 to 0.97 (FP64, up
+//     to 6 rows, 18 to 28 columns) and 0.88 to 0.96 (FP32, under 250 points);
+//     32 columns, taller and larger tiles 1.0 to 2.1.  Odd widths copy value by
+//     value: 17 columns in between 0.77 to 1.2, on odd grids with several
+//     rounds 0.74 to 0.93 (FP32 up to 6 rows 1.2 to 2.0, 32 rows 1.4 to 1.6),
+//     FP64 where it
+//     holds under 0.3 of the one-column pass's columns 0.72 to 1.2.
+//   8 or 16 columns, 6 or 8 rows (in registers): 0.95 to 1.45.  4, 5 and 7 rows
+//     (rolled loops): 0.95 to 1.4, in between 0.90 to 0.93.  1 and 2 rows, and 3
+//     rows of 16 columns: 0.78 to 1.07, FP32 with six rounds and more 1.04 to
+//     1.45.  (270 x 130 and 90 x 45, a pass of one task's latency, go down to
+//     0.85 in mixed solves at every one of these heights.)
+//     16 rows and more (staged): 0.92 to 1.5 with all tasks resident, in
+//     between 0.74 to 1.06, with several rounds 0.95 to 1.76 where it holds 0.4
+//     of the one-column pass's columns and 0.81 to 1.33 where less.
+//     9 to 15 rows (staged, too few warps fit): 0.74 to 1.3.
+//   Narrower than their segment (3, 5, 12, 14 and 15 columns): 0.64 to 1.4, most
+//     of them below 1 from 592 x 344 on: the one-column pass.
+template <typename V>
+static int pair_pass_pays(const Tiling &T, bool &pays) {
+  const TileGeom &tg = T.tg;
+  const bool fp64 = sizeof(V) == 8, wide = tg.wseg == 32;
+  pays = false;
+  if (tg.hmax > kPairMaxRows) return SEVP_OK;
+  if (!wide && (tg.tm != tg.wseg || (tg.hmax > kPairRegRows && tg.hmax < 16))) return SEVP_OK;
+  long long warps2 = 0;  // resident warps of the two-column pass
+  int slots = 0;         // resident CTAs of the one-column pass
+  int s = tile_pair_resident<V>(tg, warps2);
+  if (!s) s = one_column_slots<V, double, true, true, true>(tg, slots);
+  if (s) return s;
+  const long long tasks2 = (long long)tg.ty * pair_cols(tg);
+  const long long tasks1 = (long long)tile_warps(tg), warps1 = (long long)slots * kTileWarps;
+  const bool fits2 = tasks2 <= warps2, fits1 = tasks1 <= warps1;
+  // whether it holds at least tenths / 10 of the one-column pass's columns
+  auto holds = [&](int tenths) { return 10 * warps2 * tasks1 >= tenths * warps1 * tasks2; };
+  if (wide) {
+    const bool odd = tg.tm % 2 != 0;
+    if (fits2)
+      pays = true;
+    else if (fits1)
+      pays = !odd && (tg.tm == 32 || (fp64 ? tg.hmax > 6 : tg.tm * tg.hmax >= 250));
+    else if (odd && tg.nx % 2 != 0)
+      pays = (!fp64 && tg.hmax <= 6) || (tg.hmax >= 16 && holds(4));
+    else
+      pays = !(odd && fp64) || holds(3);
+  } else if (tg.hmax < 3 || (tg.hmax == 3 && tg.wseg == 16)) {
+    pays = !fp64 && tasks2 >= 6 * warps2;
+  } else if (tg.hmax <= kPairRegRows) {
+    pays = fits2 || !fits1 || tg.hmax == 6 || tg.hmax == 8;
+  } else {
+    pays = fits2 || (!fits1 && holds(4));
+  }
+  return SEVP_OK;
 }
 
 // Dispatch: symmetric-coefficient variant when the operator is symmetric;
@@ -1294,8 +1368,16 @@ static int launch_tile(sevp_ctx *ctx, const Tiling &T, V *r, const V *q, V *z, S
       return launch_tile_k<V, MixMat, UPDATE, DOTS, false>(ctx, T, mm, r, q, z, st, ticket_slot);
     }
   }
-  if (ctx->sym && ctx->pass_b_kernel == SEVP_PASS_B_PAIRS && pair_pass_pays(T.tg))
-    return launch_tile_pair<V, UPDATE, DOTS>(ctx, T, r, q, z, st, ticket_slot);
+  if (ctx->sym && ctx->pass_b_kernel == SEVP_PASS_B_PAIRS) {
+    signed char &choice = T.pair_choice[sizeof(V) == 8];
+    if (choice < 0) {
+      bool pays = false;
+      const int s = pair_pass_pays<V>(T, pays);
+      if (s) return s;
+      choice = pays;
+    }
+    if (choice) return launch_tile_pair<V, UPDATE, DOTS>(ctx, T, r, q, z, st, ticket_slot);
+  }
   if (ctx->sym)
     return launch_tile_k<V, double, UPDATE, DOTS, true>(ctx, T, T.d_mats, r, q, z, st, ticket_slot);
   return launch_tile_k<V, double, UPDATE, DOTS, false>(ctx, T, T.d_mats, r, q, z, st, ticket_slot);
@@ -1540,6 +1622,8 @@ extern "C" int sevp_set_resume_check(sevp_ctx *ctx, double max_rel_dev) {
 }
 
 extern "C" int sevp_pass_b_kernel_used(const sevp_ctx *ctx) { return ctx ? ctx->pass_b_used : -1; }
+
+extern "C" int sevp_tile_kernel_used(const sevp_ctx *ctx) { return ctx ? ctx->tile_used : -1; }
 
 extern "C" int sevp_set_full_coefficients(sevp_ctx *ctx, int force) {
   if (!ctx) return SEVP_BAD_ARG;

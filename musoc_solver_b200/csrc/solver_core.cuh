@@ -707,6 +707,8 @@ constexpr int kPairRegRows = 8;
 constexpr int kPairMaxRows = 32;
 template <typename V>
 int tile_pair_launch(const PairLaunch<V> &L);
-
+// Warps of the pass (one task each) that the device holds at once.
+template <typename V>
+int tile_pair_resident(const TileGeom &tg, long long &warps);
 
 }  // namespace sevp

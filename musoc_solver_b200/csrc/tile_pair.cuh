@@ -615,56 +615,63 @@ __global__ void __launch_bounds__(kPairWarps * 32, 2)
   }
 }
 
+// Resident CTAs by CTA size (in warps), and the size with the most resident
+// warps (0: not asked yet).
+struct PairFit {
+  int slots[kPairWarps + 1] = {};
+  int best = 0, sms = 0;
+};
+// Of one kernel, per sub-block count (its shared memory depends on nothing
+// else).
+template <typename V, int W, int HM, bool UPDATE, bool DOTS>
+int pair_fit(int nbmax, PairFit &fit) {
+  auto kern = k_tile_pair<V, W, HM, UPDATE, DOTS>;
+  static std::mutex mu;
+  static PairFit fits[kPairMaxRows + 1];
+  std::lock_guard<std::mutex> lock(mu);
+  PairFit &f = fits[nbmax];
+  if (!f.best) {
+    const size_t per_warp = pair_smem_per_warp<V, W, HM>(nbmax);
+    PairFit found;
+    int dev = 0, optin = 0;
+    SEVP_CUDA_TRY(cudaGetDevice(&dev));
+    SEVP_CUDA_TRY(cudaDeviceGetAttribute(&found.sms, cudaDevAttrMultiProcessorCount, dev));
+    SEVP_CUDA_TRY(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+    const size_t room = (size_t)optin - 1024;  // static shared memory of the sums
+    SEVP_CUDA_TRY(
+        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)room));
+    for (int w = kPairWarps; w >= 1; --w) {
+      int per_sm = 0;
+      if (per_warp * w > room) continue;
+      SEVP_CUDA_TRY(
+          cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, w * 32, per_warp * w));
+      found.slots[w] = per_sm * found.sms;
+      if (found.slots[w] * w > found.slots[found.best] * found.best) found.best = w;
+    }
+    if (!found.best) {
+      sevp_internal_set_message("tile pass: a warp's rows do not fit the shared memory");
+      return SEVP_BAD_ARG;
+    }
+    f = found;
+  }
+  fit = f;
+  return SEVP_OK;
+}
+
 template <typename V, int W, int HM, bool UPDATE, bool DOTS>
 int tile_pair_launch_k(const PairLaunch<V> &L) {
   auto kern = k_tile_pair<V, W, HM, UPDATE, DOTS>;
   const TileGeom &tg = L.tg;
   const size_t per_warp = pair_smem_per_warp<V, W, HM>(tg.nbmax);
-  // resident CTAs by CTA size (in warps), per sub-block count (the shared
-  // memory depends on nothing else)
-  struct Fit {
-    int slots[kPairWarps + 1] = {};
-    int best = 0;  // the CTA size with the most resident warps
-  };
-  static std::mutex mu;
-  static Fit fits[kPairMaxRows + 1];
-  static int sms = 0;
-  Fit fit;
-  int use_sms;
-  {
-    std::lock_guard<std::mutex> lock(mu);
-    Fit &f = fits[tg.nbmax];
-    if (!f.best) {
-      int dev = 0, optin = 0;
-      SEVP_CUDA_TRY(cudaGetDevice(&dev));
-      SEVP_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-      SEVP_CUDA_TRY(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-      const size_t room = (size_t)optin - 1024;  // static shared memory of the sums
-      SEVP_CUDA_TRY(
-          cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)room));
-      Fit found;
-      for (int w = kPairWarps; w >= 1; --w) {
-        int per_sm = 0;
-        if (per_warp * w > room) continue;
-        SEVP_CUDA_TRY(
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, w * 32, per_warp * w));
-        found.slots[w] = per_sm * sms;
-        if (found.slots[w] * w > found.slots[found.best] * found.best) found.best = w;
-      }
-      if (!found.best) {
-        sevp_internal_set_message("tile pass: a warp's rows do not fit the shared memory");
-        return SEVP_BAD_ARG;
-      }
-      f = found;
-    }
-    fit = f, use_sms = sms;
-  }
+  PairFit fit;
+  const int s = pair_fit<V, W, HM, UPDATE, DOTS>(tg.nbmax, fit);
+  if (s) return s;
   const long long ntasks = (long long)tg.ty * pair_cols(tg);
   // few tasks: fewer warps per CTA, so that they spread over the SMs, where
   // all tasks are then resident at once (a second round doubles the pass: 16 x
   // 16 tiles at 592 x 344, FP64, 220 tasks on 148 one-warp CTAs: 45 us, on 220:
   // 27 us)
-  int warps = (int)std::min<long long>(fit.best, std::max<long long>(1, ntasks / use_sms));
+  int warps = (int)std::min<long long>(fit.best, std::max<long long>(1, ntasks / fit.sms));
   if ((long long)fit.slots[warps] * warps < ntasks) warps = fit.best;
   const long long want = std::min<long long>((ntasks + warps - 1) / warps, fit.slots[warps]);
   const unsigned blocks =
@@ -696,18 +703,39 @@ int tile_pair_launch_w(const PairLaunch<V> &L) {
   return tile_pair_launch_k<V, W, HM, false, false>(L);
 }
 
-template <typename V, int HM>
-int tile_pair_launch_h(const PairLaunch<V> &L) {
-  if (L.tg.wseg == 8) return tile_pair_launch_w<V, 8, HM>(L);
-  if (L.tg.wseg == 16) return tile_pair_launch_w<V, 16, HM>(L);
-  return tile_pair_launch_w<V, 32, HM>(L);
+// Calls f with the tiling's lane segment and row instantiation.
+template <int HM, class F>
+int pair_dispatch_w(const TileGeom &tg, F &&f) {
+  using std::integral_constant;
+  const integral_constant<int, HM> hm;
+  if (tg.wseg == 8) return f(integral_constant<int, 8>(), hm);
+  if (tg.wseg == 16) return f(integral_constant<int, 16>(), hm);
+  return f(integral_constant<int, 32>(), hm);
 }
+template <class F>
+int pair_dispatch(const TileGeom &tg, F &&f) {
+  if (tg.hmax <= 6) return pair_dispatch_w<6>(tg, f);
+  if (tg.hmax <= 8) return pair_dispatch_w<8>(tg, f);
+  if (tg.hmax <= 16) return pair_dispatch_w<16>(tg, f);
+  return pair_dispatch_w<32>(tg, f);
+}
+
 template <typename V>
 int tile_pair_launch_any(const PairLaunch<V> &L) {
-  if (L.tg.hmax <= 6) return tile_pair_launch_h<V, 6>(L);
-  if (L.tg.hmax <= 8) return tile_pair_launch_h<V, 8>(L);
-  if (L.tg.hmax <= 16) return tile_pair_launch_h<V, 16>(L);
-  return tile_pair_launch_h<V, 32>(L);
+  return pair_dispatch(L.tg, [&](auto w, auto hm) {
+    return tile_pair_launch_w<V, decltype(w)::value, decltype(hm)::value>(L);
+  });
+}
+
+template <typename V>
+int tile_pair_resident_any(const TileGeom &tg, long long &warps) {
+  return pair_dispatch(tg, [&](auto w, auto hm) {
+    PairFit fit;
+    const int s =
+        pair_fit<V, decltype(w)::value, decltype(hm)::value, true, true>(tg.nbmax, fit);
+    warps = (long long)fit.slots[fit.best] * fit.best;
+    return s;
+  });
 }
 
 }  // namespace sevp

@@ -413,6 +413,10 @@ class SevpSolver:
         the first."""
         return int(N.lib().sevp_pass_b_kernel_used(self.h))
 
+    def tile_kernel_used(self) -> int:
+        """Kernel of the last tile pass of any kind and precision (test hook)."""
+        return int(N.lib().sevp_tile_kernel_used(self.h))
+
     def pass_a(self, z, pold, beta: float):
         """One stencil pass: (p, q, p.q) with p = z + beta p_old, q = A p."""
         pnew = self.torch.empty_like(z)
