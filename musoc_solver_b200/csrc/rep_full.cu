@@ -13,6 +13,7 @@
 // across matrix elements (MATINV, GEMM); the sequential structure of the
 // method (rows, blocks) is kept.
 #include <algorithm>
+#include <map>
 #include <mutex>
 #include <vector>
 
@@ -685,6 +686,37 @@ __global__ void k_periodic_cols(double *x, int i2, int j2) {
 }
 
 // ------------------------------------------------------------ host side
+// Whether the current device can hold the marching cluster (a device may
+// have fewer SMs free in one cluster than it takes).  The shared-memory
+// opt-in and the answer belong to the device; the last shape is kept.
+static int march_cluster_fits(size_t smem, int threads, bool &fits) {
+  struct Fit {
+    size_t smem = 0;
+    int threads = 0;
+    bool fits = false;
+  };
+  static std::mutex mu;
+  static std::map<int, Fit> by_device;
+  int dev = 0;
+  SEVP_CUDA_TRY(cudaGetDevice(&dev));
+  std::lock_guard<std::mutex> lock(mu);
+  Fit &f = by_device[dev];
+  if (f.threads == 0)
+    SEVP_CUDA_TRY(cudaFuncSetAttribute(
+        k_march_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
+  if (f.threads != threads || f.smem != smem) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(kMarchCtas);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    int n = 0;
+    SEVP_CUDA_TRY(cudaOccupancyMaxActiveClusters(&n, k_march_cluster, &cfg));
+    f.smem = smem, f.threads = threads, f.fits = n > 0;
+  }
+  fits = f.fits;
+  return SEVP_OK;
+}
+
 int dev_march_solve(const MarchArgs &a, cudaStream_t st) {
   // the cluster where a column has a thread, the blocks' rows fit its shared
   // memory, and H's zeroed columns cover the ghosts (the reference's shapes)
@@ -692,16 +724,15 @@ int dev_march_solve(const MarchArgs &a, cudaStream_t st) {
   const size_t smem = march_smem_doubles(a.m2, a.nblk, nper) * sizeof(double);
   if (a.m2 >= 2 && a.m2 <= kMarchMaxCols && a.hzero >= a.m2 + 2 &&
       (!a.periodic || a.gi0 == a.m2 + 2) && smem <= (size_t)220 * 1024) {
-    static std::once_flag once;
-    static cudaError_t err = cudaSuccess;
-    std::call_once(once, [] {
-      err = cudaFuncSetAttribute(k_march_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 220 * 1024);
-    });
-    SEVP_CUDA_TRY(err);
-    k_march_cluster<<<kMarchCtas, ceil_div(a.m2, 32) * 32, smem, st>>>(a, nper);
-    SEVP_CUDA_TRY(cudaGetLastError());
-    return SEVP_OK;
+    const int threads = ceil_div(a.m2, 32) * 32;
+    bool fits = false;
+    const int s = march_cluster_fits(smem, threads, fits);
+    if (s) return s;
+    if (fits) {
+      k_march_cluster<<<kMarchCtas, threads, smem, st>>>(a, nper);
+      SEVP_CUDA_TRY(cudaGetLastError());
+      return SEVP_OK;
+    }
   }
   int threads = std::min(1024, std::max(32, ((a.m2 + 31) / 32) * 32));
   k_march_solve<<<1, threads, 0, st>>>(a);

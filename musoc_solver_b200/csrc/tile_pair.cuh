@@ -621,20 +621,21 @@ struct PairFit {
   int slots[kPairWarps + 1] = {};
   int best = 0, sms = 0;
 };
-// Of one kernel, per sub-block count (its shared memory depends on nothing
-// else).
+// Of one kernel on the current device, per sub-block count (its shared memory
+// depends on nothing else).
 template <typename V, int W, int HM, bool UPDATE, bool DOTS>
 int pair_fit(int nbmax, PairFit &fit) {
   auto kern = k_tile_pair<V, W, HM, UPDATE, DOTS>;
   static std::mutex mu;
-  static PairFit fits[kPairMaxRows + 1];
+  static std::map<int, std::array<PairFit, kPairMaxRows + 1>> fits;
+  int dev = 0;
+  SEVP_CUDA_TRY(cudaGetDevice(&dev));
   std::lock_guard<std::mutex> lock(mu);
-  PairFit &f = fits[nbmax];
+  PairFit &f = fits[dev][nbmax];
   if (!f.best) {
     const size_t per_warp = pair_smem_per_warp<V, W, HM>(nbmax);
     PairFit found;
-    int dev = 0, optin = 0;
-    SEVP_CUDA_TRY(cudaGetDevice(&dev));
+    int optin = 0;
     SEVP_CUDA_TRY(cudaDeviceGetAttribute(&found.sms, cudaDevAttrMultiProcessorCount, dev));
     SEVP_CUDA_TRY(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
     const size_t room = (size_t)optin - 1024;  // static shared memory of the sums

@@ -1,5 +1,7 @@
 // Two-column tile pass (tile_pair.cuh) on vectors of type double.
 #include <algorithm>
+#include <array>
+#include <map>
 #include <mutex>
 #include <type_traits>
 
