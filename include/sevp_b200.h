@@ -338,6 +338,13 @@ int sevp_pass_a_f32(sevp_ctx *ctx, const float *z, const float *pold, double bet
                     float *q, double *pq_out);
 int sevp_pass_a_f64(sevp_ctx *ctx, const double *z, const double *pold, double beta,
                     double *pnew, double *q, double *pq_out);
+/* One preconditioner pass of an iteration on caller device buffers: r -= alpha
+ * q in place, z = M^-1 r, and r.z and r.r through rz_out and rr_out.  Test
+ * hook; not part of the reference interface. */
+int sevp_pass_b_f32(sevp_ctx *ctx, double alpha, float *r, const float *q, float *z,
+                    double *rz_out, double *rr_out);
+int sevp_pass_b_f64(sevp_ctx *ctx, double alpha, double *r, const double *q, double *z,
+                    double *rz_out, double *rr_out);
 
 int sevp_set_full_coefficients(sevp_ctx *ctx, int force);
 /* Device bytes held by the tile influence data (block-Jacobi tiling). */

@@ -3225,3 +3225,35 @@ extern "C" int sevp_pass_a_f64(sevp_ctx *ctx, const double *z, const double *pol
                                double *pnew, double *q, double *pq_out) {
   return pass_a_step(ctx, z, pold, beta, pnew, q, pq_out);
 }
+
+// One pass B on caller buffers.
+__global__ void k_state_pass_b(SolveState *st, double alpha) {
+  SolveState s{};
+  s.alpha = alpha;
+  s.rz = 1.0;
+  s.max_iter = 1 << 30;
+  s.status = SEVP_OK;
+  *st = s;
+}
+
+template <typename V>
+static int pass_b_step(sevp_ctx *ctx, double alpha, V *r, const V *q, V *z, double *rz_out,
+                       double *rr_out) {
+  if (!ctx || !ctx->have_op || !r || !q || !z) return SEVP_BAD_ARG;
+  k_state_pass_b<<<1, 1, 0, ctx->stream>>>(ctx->st, alpha);
+  int s = precondition_pass<V, true, true>(ctx, r, q, z);
+  if (!s) s = read_state(ctx);
+  if (s) return s;
+  if (rz_out) *rz_out = ctx->h_st->rz_next;
+  if (rr_out) *rr_out = ctx->h_st->rr;
+  return ctx->h_st->status;
+}
+
+extern "C" int sevp_pass_b_f32(sevp_ctx *ctx, double alpha, float *r, const float *q, float *z,
+                               double *rz_out, double *rr_out) {
+  return pass_b_step(ctx, alpha, r, q, z, rz_out, rr_out);
+}
+extern "C" int sevp_pass_b_f64(sevp_ctx *ctx, double alpha, double *r, const double *q, double *z,
+                               double *rz_out, double *rr_out) {
+  return pass_b_step(ctx, alpha, r, q, z, rz_out, rr_out);
+}

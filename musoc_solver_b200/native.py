@@ -130,6 +130,8 @@ _SIGS = {
     "sevp_set_resume_check": ([P, C.c_double], C.c_int),
     "sevp_pass_a_f32": ([P, P, P, C.c_double, P, P, P], C.c_int),
     "sevp_pass_a_f64": ([P, P, P, C.c_double, P, P, P], C.c_int),
+    "sevp_pass_b_f32": ([P, C.c_double, P, P, P, P, P], C.c_int),
+    "sevp_pass_b_f64": ([P, C.c_double, P, P, P, P, P], C.c_int),
     "sevp_set_schwarz": ([P, C.c_int], C.c_int),
     "sevp_schwarz_shift": ([P], C.c_int),
     "sevp_record_coefficients": ([P, C.c_int], C.c_int),

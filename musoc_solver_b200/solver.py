@@ -427,6 +427,15 @@ class SevpSolver:
                    C.byref(pq)), "sevp_pass_a")
         return pnew, q, pq.value
 
+    def pass_b(self, alpha: float, r, q):
+        """One preconditioner pass: r -= alpha q in place; (z, r.z, r.r)."""
+        z = self.torch.empty_like(r)
+        rz, rr = C.c_double(), C.c_double()
+        fn = N.lib().sevp_pass_b_f64 if r.dtype == self.torch.float64 else N.lib().sevp_pass_b_f32
+        N.check(fn(self.h, float(alpha), N.ptr(r), N.ptr(q), N.ptr(z), C.byref(rz), C.byref(rr)),
+                "sevp_pass_b")
+        return z, rz.value, rr.value
+
     def precondition(self, r):
         z = self.torch.empty_like(r)
         fn = N.lib().sevp_precondition if r.dtype == self.torch.float64 else N.lib().sevp_precondition_f32
