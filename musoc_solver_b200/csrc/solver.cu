@@ -2243,7 +2243,7 @@ static int graph_loop(sevp_ctx *ctx, bool graph, const void *const (&key)[5], in
     const double left_log = log(ctx->h_st->tol2 * ctx->h_st->bb / ctx->h_st->rr);
     if (pcg_iters && !ctx->prof && it0 > 0 && done_log < -1.0 && left_log < 0.0) {
       const double left = left_log / done_log * it0;  // iterations at the rate so far
-      batch = std::max(1, std::min(16, (int)(0.8 * left / check_every)));
+      batch = (int)std::max(1.0, std::min(16.0, 0.8 * left / check_every));
     }
   }
   return SEVP_OK;
