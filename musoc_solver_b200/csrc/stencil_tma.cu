@@ -57,9 +57,9 @@ struct Stage {
                             kOff_al = kOff_at + kAT, kOff_ab = kOff_al + kAC;
   static constexpr uint32_t kBytes = kOff_al + (SYM ? 0 : 2 * kAC);
   // bytes the copies of one stage deliver (the full boxes, fill included)
-  static constexpr uint32_t kTxVectors = 2 * kBW * (kTH + 2) * sizeof(V);
-  static constexpr uint32_t kTxPlanes = kTW * kTH * 4 + (kTW + 4) * kTH * 4 +
-                                        kTW * (kTH + 1) * 4 + (SYM ? 0 : 2 * kTW * kTH * 4);
+  static constexpr uint32_t kTx = 2 * kBW * (kTH + 2) * sizeof(V) + kTW * kTH * 4 +
+                                  (kTW + 4) * kTH * 4 + kTW * (kTH + 1) * 4 +
+                                  (SYM ? 0 : 2 * kTW * kTH * 4);
 };
 
 struct Maps {
@@ -92,62 +92,17 @@ __global__ void __launch_bounds__(kThreads, 2)
                  const V *__restrict__ pold, const float *__restrict__ ar_g, V *pnew, V *q,
                  V *__restrict__ x, SolveState *st, double *partials, unsigned *ticket) {
   using S = Stage<V, SYM>;
-  pdl_trigger();
+  // The state is read before anything else is set up.  With the planes' copies
+  // ahead of the wait, or the state read after the barriers, an FP64 launch at
+  // 3600 x 2400 took 98 us instead of 89 (the same occupancy, 128 instead of
+  // 126 registers), more than the early copies gained on any grid.
+  pdl_wait();
+  if (st->done) return;
   extern __shared__ __align__(128) unsigned char sm_raw[];
   __shared__ __align__(8) uint64_t full[STAGES];
   const uint32_t sbase = (smem_u32(sm_raw) + 127u) & ~127u;
   unsigned char *sgen = sm_raw + (sbase - smem_u32(sm_raw));
   const int tid = threadIdx.x;
-  const int nx = g.nx, ny = g.ny;
-  const int TX = (nx + kTW - 1) / kTW, TY = (ny + kTH - 1) / kTH, ntile = TX * TY;
-  if (tid == 0) {
-    for (int s = 0; s < STAGES; ++s) mbar_init(smem_u32(&full[s]), 2);
-    tma::fence_mbar_init();
-  }
-  __syncthreads();
-  // the copies of this CTA's k-th tile: the planes, then the vectors (one
-  // arrival each on the stage's barrier)
-  auto issue_planes = [&](int k) {
-    const int t = blockIdx.x + k * gridDim.x;
-    const int x0 = (t % TX) * kTW, j0 = (t / TX) * kTH;
-    const uint32_t st0 = sbase + (uint32_t)(k % STAGES) * S::kBytes;
-    const uint32_t bar = smem_u32(&full[k % STAGES]);
-    // the stage's previous tile was read and written through the generic
-    // proxy (ordered before this thread by the CTA barrier)
-    tma::fence_proxy_async();
-    mbar_expect_tx(bar, S::kTxPlanes);
-    tma::load_2d(st0 + S::kOff_ac, &maps.ac, x0, j0, bar);
-    tma::load_2d(st0 + S::kOff_ar, &maps.ar, x0 - 4, j0, bar);
-    tma::load_2d(st0 + S::kOff_at, &maps.at, x0, j0 - 1, bar);
-    if (!SYM) {
-      tma::load_2d(st0 + S::kOff_al, &maps.al, x0, j0, bar);
-      tma::load_2d(st0 + S::kOff_ab, &maps.ab, x0, j0, bar);
-    }
-  };
-  auto issue_vectors = [&](int k) {
-    const int t = blockIdx.x + k * gridDim.x;
-    const int x0 = (t % TX) * kTW, j0 = (t / TX) * kTH;
-    const uint32_t st0 = sbase + (uint32_t)(k % STAGES) * S::kBytes;
-    const uint32_t bar = smem_u32(&full[k % STAGES]);
-    mbar_expect_tx(bar, S::kTxVectors);
-    tma::load_2d(st0 + S::kOff_z, &maps.z, x0 - S::kH, j0 - 1, bar);
-    tma::load_2d(st0 + S::kOff_p, &maps.p, x0 - S::kH, j0 - 1, bar);
-  };
-  const int nmine = blockIdx.x < ntile ? (ntile - 1 - blockIdx.x) / gridDim.x + 1 : 0;
-  // the operator's planes are on their way before the kernel ahead has ended
-  if (tid == 0)
-    for (int k = 0; k < STAGES - 1 && k < nmine; ++k) issue_planes(k);
-  pdl_wait();
-  if (st->done) {
-    if (tid == 0)
-      for (int k = 0; k < STAGES - 1 && k < nmine; ++k) {
-        mbar_expect_tx(smem_u32(&full[k]), 0);
-        mbar_wait(smem_u32(&full[k]), 0);
-      }
-    return;
-  }
-  if (tid == 0)
-    for (int k = 0; k < STAGES - 1 && k < nmine; ++k) issue_vectors(k);
   const V beta = (V)st->beta;
   const bool first = st->beta == 0.0;
   // the pending step of the iteration before: x += alpha p_old on the own
@@ -156,15 +111,46 @@ __global__ void __launch_bounds__(kThreads, 2)
   const bool step = x != nullptr && st->x_pend;
   const bool x_init = st->x_init;
   const V alpha = (V)st->alpha;
+  const int nx = g.nx, ny = g.ny;
+  const int TX = (nx + kTW - 1) / kTW, TY = (ny + kTH - 1) / kTH, ntile = TX * TY;
+  if (tid == 0) {
+    for (int s = 0; s < STAGES; ++s) mbar_init(smem_u32(&full[s]), 1);
+    tma::fence_mbar_init();
+  }
+  __syncthreads();
+  auto issue = [&](int k) {  // the copies of this CTA's k-th tile
+    const int t = blockIdx.x + k * gridDim.x;
+    if (t >= ntile) return;
+    const int x0 = (t % TX) * kTW, j0 = (t / TX) * kTH;
+    const uint32_t st0 = sbase + (uint32_t)(k % STAGES) * S::kBytes;
+    const uint32_t bar = smem_u32(&full[k % STAGES]);
+    // the stage's previous tile was read and written through the generic
+    // proxy (ordered before this thread by the CTA barrier)
+    tma::fence_proxy_async();
+    mbar_expect_tx(bar, S::kTx);
+    tma::load_2d(st0 + S::kOff_z, &maps.z, x0 - S::kH, j0 - 1, bar);
+    tma::load_2d(st0 + S::kOff_p, &maps.p, x0 - S::kH, j0 - 1, bar);
+    tma::load_2d(st0 + S::kOff_ac, &maps.ac, x0, j0, bar);
+    tma::load_2d(st0 + S::kOff_ar, &maps.ar, x0 - 4, j0, bar);
+    tma::load_2d(st0 + S::kOff_at, &maps.at, x0, j0 - 1, bar);
+    if (!SYM) {
+      tma::load_2d(st0 + S::kOff_al, &maps.al, x0, j0, bar);
+      tma::load_2d(st0 + S::kOff_ab, &maps.ab, x0, j0, bar);
+    }
+  };
+  const int nmine = blockIdx.x < ntile ? (ntile - 1 - blockIdx.x) / gridDim.x + 1 : 0;
+  if (tid == 0)
+    for (int k = 0; k < STAGES - 1 && k < nmine; ++k) issue(k);
   double acc[2] = {0.0, 0.0};
   bool failed = false;
   int kfail = nmine;  // first tile whose wait gave up
   const int tx = tid % kTW, ty = tid / kTW;
   for (int k = 0; k < nmine; ++k) {
-    if (tid == 0 && k + STAGES - 1 < nmine) {
-      issue_planes(k + STAGES - 1);
-      issue_vectors(k + STAGES - 1);
-    }
+    if (tid == 0 && k + STAGES - 1 < nmine) issue(k + STAGES - 1);
+    // the tile pass may start beside the CTAs' last tiles; triggered from the
+    // start its waiting CTAs took room from this pass's (3600 x 2400 FP64 solve
+    // 11.25 against 11.11 ms)
+    if (k == nmine - 1) pdl_trigger();
     const int t = blockIdx.x + k * gridDim.x;
     const int x0 = (t % TX) * kTW, j0 = (t / TX) * kTH;
     unsigned char *sp = sgen + (size_t)(k % STAGES) * S::kBytes;
