@@ -465,8 +465,10 @@ __global__ void __launch_bounds__(kPairWarps * 32, 2)
         }
       }
       // Row k's coefficients and right-hand side, converted, and its
-      // reciprocals of AT: taken one row ahead of the march, so that only the
-      // shuffles, one multiply-add and the quotient are on its chain.
+      // reciprocals of AT.  Taken at the row's use: one row ahead, the copies
+      // they made cost more than the shorter chain gained at every height
+      // (FP32 pass, 64 x 720 x 360 members, 16 x 6 tiles: 277 against 262 us; 24
+      // x 24 tiles at 2400 x 1500: 236 against 218 us).
       struct RowC {
         double s0, s1, f0, f1, e0, e1, w0, n0, n1, i0, i1, p0, p1;
       };
@@ -502,10 +504,9 @@ __global__ void __launch_bounds__(kPairWarps * 32, 2)
       {
         double zb0 = 0.0, zb1 = 0.0, zc0 = 0.0, zc1 = 0.0, q0, q1;
         int t = 0, kb = 0, ke = sub_start(1, hh, nb) - 1;
-        RowC c = take(0);
 #pragma unroll 1
         for (int k = 0; k < hh; ++k) {
-          const RowC cn = take(min(k + 1, hh - 1));
+          const RowC c = take(k);
           if (k == kb) {
             zc0 = zc1 = 0.0;
             zin[t * 32] = make_double2(zb0, zb1);
@@ -515,7 +516,6 @@ __global__ void __launch_bounds__(kPairWarps * 32, 2)
           if (last) rho[t * 32] = make_double2(q0, q1);
           zb0 = zc0, zb1 = zc1;
           if (!last) zc0 = march_quot<V>(q0, c.n0, c.i0), zc1 = march_quot<V>(q1, c.n1, c.i1);
-          c = cn;
           if (__any_sync(0xffffffffu, fix)) {
             __syncwarp();
             *dv2 = make_double2(q0, q1);
@@ -580,10 +580,9 @@ __global__ void __launch_bounds__(kPairWarps * 32, 2)
         }
         double zc0 = v0, zc1 = v1, q0, q1;
         const int k_lo = __reduce_min_sync(0xffffffffu, kb), k_hi = __reduce_max_sync(0xffffffffu, ke);
-        RowC c = take(k_lo);
 #pragma unroll 1
         for (int k = k_lo; k <= k_hi; ++k) {
-          const RowC cn = take(min(k + 1, hh - 1));
+          const RowC c = take(k);
           const bool in = on && k >= kb && k <= ke;
           if (in) {
             const V u0 = (V)zc0, u1 = (V)zc1;
@@ -598,7 +597,6 @@ __global__ void __launch_bounds__(kPairWarps * 32, 2)
             zb0 = zc0, zb1 = zc1;
             zc0 = march_quot<V>(q0, c.n0, c.i0), zc1 = march_quot<V>(q1, c.n1, c.i1);
           }
-          c = cn;
         }
         vn0 = v0, vn1 = v1;
       }
