@@ -1283,30 +1283,32 @@ static int launch_tile_pair(sevp_ctx *ctx, const Tiling &T, V *r, const V *q, V 
 }
 
 // Whether the two-column pass is the faster one for a tiling.  Numbers: whole
-// solves, one-column time over two-column time on one B200 (FP64 and mixed),
-// sixteen grids from 90 x 45 to 3600 x 2400, 103 tile shapes.
+// solves, one-column time over two-column time on one B200 (least, median and
+// largest of FP64 and mixed), 103 tile shapes on sixteen grids from 90 x 45 to
+// 3600 x 2400.
 //
-// Its warps hold two tasks' columns, so it takes half as many, but they need
-// more registers and shared memory: it holds 1/2 to 1/6 of the one-column
-// pass's warps.  While all its tasks are resident it is the faster one; where
-// they take a second round and the one-column pass's still fit one, the
-// second round costs more than the two columns gain on small tiles.
-//   32-lane segments (17 to 32 columns): 1.0 to 2.5 with all tasks resident
-//     and with several rounds on both sides, in between 0.86 to 0.97 (FP64, up
-//     to 6 rows, 18 to 28 columns) and 0.88 to 0.96 (FP32, under 250 points);
-//     32 columns, taller and larger tiles 1.0 to 2.1.  Odd widths copy value by
-//     value: 17 columns in between 0.77 to 1.2, on odd grids with several
-//     rounds 0.74 to 0.93 (FP32 up to 6 rows 1.2 to 2.0, 32 rows 1.4 to 1.6),
-//     FP64 where it
-//     holds under 0.3 of the one-column pass's columns 0.72 to 1.2.
-//   8 or 16 columns, 6 or 8 rows (in registers): 0.95 to 1.45.  4, 5 and 7 rows
-//     (rolled loops): 0.95 to 1.4, in between 0.90 to 0.93.  1 and 2 rows, and 3
-//     rows of 16 columns: 0.78 to 1.07, FP32 with six rounds and more 1.04 to
-//     1.45.  (270 x 130 and 90 x 45, a pass of one task's latency, go down to
-//     0.85 in mixed solves at every one of these heights.)
-//     16 rows and more (staged): 0.92 to 1.5 with all tasks resident, in
-//     between 0.74 to 1.06, with several rounds 0.95 to 1.76 where it holds 0.4
-//     of the one-column pass's columns and 0.81 to 1.33 where less.
+// A warp of it holds two tasks' columns, so it takes half as many, but they
+// need more registers and shared memory: the device holds 1/2 to 1/6 as many
+// of them.  While all its tasks are resident it is the faster one.  Between: its
+// tasks take a second round while the one-column pass's fit one, which costs
+// more than the two columns gain on small tiles.
+//   32-lane segments (17 to 32 columns): all resident 0.97, 1.64, 3.0; several
+//     rounds on both sides 0.96, 1.66, 3.6.  Between: FP64 up to 6 rows 0.87,
+//     1.00, 1.08, FP32 under 250 points 0.87, 0.99, 1.16: the one-column pass;
+//     taller and larger tiles, and 32 columns, 0.98, 1.45, 2.5.
+//     17 columns (an odd width copies value by value, and half the lanes idle):
+//     between 0.80, 1.00, 1.41, FP64 that holds under 0.3 of the one-column
+//     pass's columns 0.76, 0.96, 1.31, odd grids 0.77, 1.03, 1.20 except FP32 up to
+//     6 rows and the tallest tiles 1.18, 1.46, 2.08: the one-column pass for all
+//     but these.  (19, 23 and 27 columns run as the even widths do.)
+//   8 or 16 columns, 6 or 8 rows (in registers): 0.96, 1.12, 1.58.  4, 5 and 7
+//     rows and 8 x 3 (rolled loops): 0.95, 1.10, 1.39, between 0.90, 0.97, 1.01.
+//     1 and 2 rows and 16 x 3: all resident 0.92, 1.03, 1.15, FP32 with six rounds
+//     and more 1.05, 1.23, 1.59, the others 0.80, 0.99, 1.09.  (270 x 130 and 90 x 45, a pass of one task's latency:
+//     0.90, 1.02, 1.12 over all these heights.)
+//     16 rows and more (staged): all resident 0.95, 1.23, 1.60, between 0.79,
+//     1.01, 1.12, several rounds 0.95, 1.28, 1.91 where it holds 0.3 of the
+//     one-column pass's columns and 0.85 to 0.90 where less.
 //     9 to 15 rows (staged, too few warps fit): 0.74 to 1.3.
 //   Narrower than their segment (3, 5, 12, 14 and 15 columns): 0.64 to 1.4, most
 //     of them below 1 from 592 x 344 on: the one-column pass.
@@ -1328,21 +1330,21 @@ static int pair_pass_pays(const Tiling &T, bool &pays) {
   // whether it holds at least tenths / 10 of the one-column pass's columns
   auto holds = [&](int tenths) { return 10 * warps2 * tasks1 >= tenths * warps1 * tasks2; };
   if (wide) {
-    const bool odd = tg.tm % 2 != 0;
+    const bool half = tg.tm == 17;
     if (fits2)
       pays = true;
     else if (fits1)
-      pays = !odd && (tg.tm == 32 || (fp64 ? tg.hmax > 6 : tg.tm * tg.hmax >= 250));
-    else if (odd && tg.nx % 2 != 0)
+      pays = !half && (tg.tm == 32 || (fp64 ? tg.hmax > 6 : tg.tm * tg.hmax >= 250));
+    else if (half && tg.nx % 2 != 0)
       pays = (!fp64 && tg.hmax <= 6) || (tg.hmax >= 16 && holds(4));
     else
-      pays = !(odd && fp64) || holds(3);
+      pays = !(half && fp64) || holds(3);
   } else if (tg.hmax < 3 || (tg.hmax == 3 && tg.wseg == 16)) {
-    pays = !fp64 && tasks2 >= 6 * warps2;
+    pays = fits2 || (!fp64 && tasks2 >= 6 * warps2);
   } else if (tg.hmax <= kPairRegRows) {
     pays = fits2 || !fits1 || tg.hmax == 6 || tg.hmax == 8;
   } else {
-    pays = fits2 || (!fits1 && holds(4));
+    pays = fits2 || (!fits1 && holds(3));
   }
   return SEVP_OK;
 }
@@ -1555,7 +1557,8 @@ extern "C" int sevp_create(sevp_ctx **out, int nx, int ny, int periodic, void *s
   ALLOC(ctx->st, sizeof(SolveState));
   ALLOC(ctx->tickets, 16 * sizeof(unsigned));
   // partial sums: enough for the larger of the stencil and tile grids
-  // stencil grid: ceil(nx / 256) x ceil(ny / rpw), rpw >= 8
+  // stencil grid: ceil(nx / 256) x ceil(ny / rpw), rpw >= 8 (stencil_rpw takes
+  // fewer rows only where five sums per CTA fit as well)
   size_t sgrid = (size_t)ceil_div(ceil_div(nx, kStencilCols), kStencilThreads / 32) * ceil_div(ny, 8);
   size_t tgrid = (size_t)ceil_div(nx, 1) * ceil_div(ny, 1) / (kTileWarps) + 1024;
   ctx->partials_n = std::max(sgrid, tgrid) * 2 + 64;
