@@ -701,8 +701,9 @@ struct PairLaunch {
   cudaStream_t stream;
   bool update, dots;
 };
-// Tile rows the kernel holds in registers (taller tiles run its rolled loops
-// on rows staged in shared memory), and the most it takes.
+// Most tile rows of the instantiations that hold full tiles in registers (6
+// and 8 rows; tiles of other heights, and taller ones, run rolled loops on rows
+// staged in shared memory), and the most rows the kernel takes.
 constexpr int kPairRegRows = 8;
 constexpr int kPairMaxRows = 32;
 template <typename V>

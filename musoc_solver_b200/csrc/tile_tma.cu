@@ -3,9 +3,10 @@
 // finish of the iteration (the pass of k_tile_short in solver.cu, operation
 // for operation: r and z come out bit-identical).
 //
-// The register kernel loads a task's rows (r, q and the planes AC, AR, AT) and, after the forward march, its influence matrices from global
-// memory, so every task waits out two memory round trips with only 16 warps
-// per SM to cover them.  Here each warp keeps a shared-memory stage of one
+// The register kernel loads a task's rows (r, q and the planes AC, AR, AT)
+// and, after the forward march, its influence matrices from global memory, so
+// every task waits out two memory round trips with only 16 warps per SM to
+// cover them.  Here each warp keeps a shared-memory stage of one
 // task: while it marches task t, the copies of task t + stride are in
 // flight.  Lane 0 issues them:
 //   - the rows, as five 2-D tensor copies of a 32 x th box (columns
